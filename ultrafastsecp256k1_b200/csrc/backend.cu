@@ -52,10 +52,8 @@ cudaError_t Backend::launch_verify(int kind, const uint8_t* m, const uint8_t* p,
     if (kind != 2 && call_items <= pair_items_[k])
         return launch_verify_pair(kind, m, p, s, n, d_gtab_, out, collect, st);
     const bool small = small_variant_[k] >= 0 && call_items <= small_items_[k];
-    if (!small && inv_group_[k] > 1) {
-        const int gi = inv_group_[k] == 64 ? 0 : 1;
-        return launch_verify_grp(inv_group_[k], kind, m, p, s, n, d_gtab_, out, collect, grp_grid_[gi][k], st);
-    }
+    if (!small && inv_group_[k] > 1)
+        return launch_verify_fp(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, sms_, st);
     const int v = small ? small_variant_[k] : variant_[k];
     return kLaunchers[v](kind, m, p, s, n, gtab_for(v), out, collect, grid_[v][k], st);
 }
@@ -309,6 +307,7 @@ Backend::~Backend() {
             if (pstream_[j]) cudaStreamDestroy(pstream_[j]);
         }
         if (d_gtab_) cudaFree(d_gtab_);
+        if (d_comb_) cudaFree(d_comb_);
         for (void*& t : gtab_w_)
             if (t) cudaFree(t);
         if (stream_) cudaStreamDestroy(stream_);
@@ -362,12 +361,13 @@ int Backend::init(int device_index) {
         return cuda_error(e, "cudaStreamCreate");
     if ((e = cudaMalloc(&d_gtab_, kGTableBytes)) != cudaSuccess) return cuda_error(e, "cudaMalloc(gtab)");
     if ((e = launch_gtable_init(d_gtab_, stream_)) != cudaSuccess) return cuda_error(e, "gtable init launch");
+    if ((e = cudaMalloc(&d_comb_, comb_table_bytes())) != cudaSuccess) return cuda_error(e, "cudaMalloc(comb)");
+    if ((e = launch_comb_init(d_comb_, stream_)) != cudaSuccess) return cuda_error(e, "generator windows launch");
     if ((e = cudaStreamSynchronize(stream_)) != cudaSuccess) return cuda_error(e, "gtable init");
     for (int v = 0; v < kVerifyVariants; ++v)
         for (int k = 0; k < 2; ++k) grid_[v][k] = std::max(1, kOccupancy[v](k)) * sms_;
     queue_grid_ = std::max(1, verify_queue_occupancy()) * sms_;
-    for (int gi = 0; gi < 2; ++gi)
-        for (int k = 0; k < 2; ++k) grp_grid_[gi][k] = std::max(1, verify_grp_occupancy(gi ? 128 : 64, k)) * sms_;
+    if ((e = verify_fp_init()) != cudaSuccess) return cuda_error(e, "verify kernel set-up");
     queue_pair_grid_ = std::max(1, verify_pair_occupancy()) * sms_;   // also the two-lane kernels' shared-memory opt-in
     load_tuning();
     // generator tables of the window widths the chosen variants use; a variant
@@ -392,7 +392,11 @@ int Backend::verify_device(int kind, const uint8_t* d_msgs, const uint8_t* d_pub
     cudaError_t e = cudaSetDevice(dev_);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
     cudaStream_t s = stream ? stream : stream_;
-    if (count < 2 * kDeviceChunk) {
+    // The FP64 kernel takes any number of items in one launch (one block per SM at
+    // a time, handed out as they finish).
+    if (count < 2 * kDeviceChunk || inv_group_[kind & 1] > 1) {
+        if (count >= 2 * kDeviceChunk)
+            if (const int rc = fault_point("verify launch")) return rc;
         e = launch_verify(kind, d_msgs, d_pubs, d_sigs, (uint32_t)count, d_out, 0, s, count);
         if (e != cudaSuccess) return cuda_error(e, "verify launch");
         clear_error();

@@ -193,7 +193,6 @@ private:
     // variant choice.
     uint32_t pair_items_[2] = {0, 0};
     int inv_group_[2] = {1, 1};
-    int grp_grid_[2][2] = {};    // [64, 128][kind] resident-grid size of the batch-inversion kernels
     // call_items: the size of the whole call this launch belongs to; the
     // small-launch variant is used only when the whole call is small (the
     // chunks of a large call run beside one another at full occupancy).
@@ -202,6 +201,7 @@ private:
     void load_tuning();
     cudaStream_t stream_ = nullptr;
     void* d_gtab_ = nullptr;
+    void* d_comb_ = nullptr;    // generator window table (isocheck.cuh)
     DevBuf msgs_, pubs_, sigs_, out_, scratch_, ops_in_;
     // host-buffer calls: kPipeSlots pinned staging slots, each with its own
     // stream, so that the CPU packs chunk k + 2 while the device verifies

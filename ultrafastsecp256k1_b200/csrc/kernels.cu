@@ -4,6 +4,7 @@
 #include "kernels.h"
 #include "verify.cuh"
 #include "dev_tables.cuh"
+#include "isocheck.cuh"
 
 namespace uf {
 
@@ -44,6 +45,56 @@ cudaError_t launch_gtable_init_w(void* d_gtab, int wbits, cudaStream_t s) {
 }
 
 cudaError_t launch_gtable_init(void* d_gtab, cudaStream_t s) { return launch_gtable_init_w(d_gtab, UF_GWIN, s); }
+
+// ------------------------------------------------- generator window table --
+__device__ __forceinline__ void store_aff(uint4* q, const Aff& A) {
+    q[0] = make_uint4(A.x.v[0], A.x.v[1], A.x.v[2], A.x.v[3]);
+    q[1] = make_uint4(A.x.v[4], A.x.v[5], A.x.v[6], A.x.v[7]);
+    q[2] = make_uint4(A.y.v[0], A.y.v[1], A.y.v[2], A.y.v[3]);
+    q[3] = make_uint4(A.y.v[4], A.y.v[5], A.y.v[6], A.y.v[7]);
+}
+
+// entry 0 of every window: 2^(16 i) G (one thread per window)
+__global__ void k_comb_base(uint4* out) {
+    const int i = threadIdx.x;
+    if (i >= kCombWindows) return;
+    Aff G;
+    gen_point(G);
+    Jac acc;
+    jac_from_aff(acc, G.x, G.y);
+    for (int k = 0; k < 16 * i; ++k) jac_dbl(acc);
+    Aff A;
+    jac_to_aff(A, acc);
+    store_aff(out + 4 * (size_t)i * kCombTab, A);
+}
+
+// entry m - 1 of window i: m 2^(16 i) G, m = 2..2^15
+__global__ void k_comb_init(uint4* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t / kCombTab, m = t % kCombTab + 1;
+    if (i >= kCombWindows || m == 1) return;
+    const uint4* q = out + 4 * (size_t)i * kCombTab;
+    const uint4 a = q[0], b = q[1], c = q[2], d = q[3];
+    const Fe x = {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}}, y = {{c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w}};
+    Jac acc;
+    jac_set_inf(acc);
+    for (int k = 31 - __clz(m); k >= 0; --k) {
+        jac_dbl(acc);
+        if ((m >> k) & 1) jac_add_aff(acc, x, y);
+    }
+    Aff A;
+    jac_to_aff(A, acc);
+    store_aff(out + 4 * (size_t)t, A);
+}
+
+size_t comb_table_bytes() { return kCombBytes; }
+
+cudaError_t launch_comb_init(void* d_comb, cudaStream_t s) {
+    uint4* out = reinterpret_cast<uint4*>(d_comb);
+    k_comb_base<<<1, 32, 0, s>>>(out);
+    k_comb_init<<<kCombWindows * kCombTab / 256, 256, 0, s>>>(out);
+    return cudaGetLastError();
+}
 
 // ---------------------------------------------------------- diagnostics --
 // op: 1 fe_mul(64->32) 2 fe_sqr(32->32) 3 fe_inv(32->32) 4 fe_sqrt(32->33)

@@ -76,13 +76,16 @@ int verify_occupancy_v9(int kind);
 int verify_occupancy_v10(int kind);
 int verify_occupancy_v11(int kind);
 
-// The same verify with block-wide batch inversion (kernels_verify_grp.cu):
-// the table, final-Z and ECDSA s inversions are shared by the `group` (64 or
-// 128) threads of a block.  `grid` resident blocks from verify_grp_occupancy,
-// which also opts the kernels in to their shared memory.
-cudaError_t launch_verify_grp(int group, int kind, const uint8_t* msgs, const uint8_t* pubs, const uint8_t* sigs,
-                              uint32_t n, const void* d_gtab, uint8_t* out, int collect, int grid, cudaStream_t s);
-int verify_grp_occupancy(int group, int kind);
+// The same verify without the key's square root, its field arithmetic on the
+// FP64 pipe (kernels_verify_fp.cu).  d_comb: the generator window table.
+// verify_fp_init opts the kernels in to their shared memory (once per device).
+cudaError_t launch_verify_fp(int kind, const uint8_t* msgs, const uint8_t* pubs, const uint8_t* sigs, uint32_t n,
+                             const void* d_gtab, const void* d_comb, uint8_t* out, int collect, int sms,
+                             cudaStream_t s);
+cudaError_t verify_fp_init();
+// Fills the generator window table (comb_table_bytes() bytes; isocheck.cuh).
+size_t comb_table_bytes();
+cudaError_t launch_comb_init(void* d_comb, cudaStream_t s);
 
 // Per-item batch operations (kernels_ops.cu); device pointers, asynchronous.
 cudaError_t launch_xonly_validate(const uint8_t* keys32, uint32_t n, uint8_t* out, int sms, cudaStream_t s);
