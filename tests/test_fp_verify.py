@@ -158,11 +158,7 @@ def fp_ctx():
         yield ctx
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("n", [1, 31, 33, 147, 149, 4737, 18945, 37887, 37888, 37889, 80001])
-def test_block_edges(fp_ctx, oracle, n):
-    """One item to two rounds of full blocks, around the block and grid sizes
-    (148 SMs, up to 256 items each), both schemes and the opaque rows."""
+def check_sizes(fp_ctx, oracle, n):
     import ultrafastsecp256k1_b200 as uf
     m = min(n, 701)
     order = np.random.default_rng(n).integers(0, m, n)
@@ -179,6 +175,14 @@ def test_block_edges(fp_ctx, oracle, n):
     tiled = np.ascontiguousarray(rows[order])
     assert L.ufsecp_gpu_ecdsa_verify_opaque_rows(fp_ctx.handle, tiled.ctypes.data, 129, n, out.ctypes.data) == 0
     assert (out == oracle.ecdsa_verify_opaque_rows(rows, 129)[order]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 33, 147, 149, 4737, 18945, 37887, 37888, 37889, 80001])
+def test_block_edges(fp_ctx, oracle, n):
+    """One item to two rounds of full blocks, around the block and grid sizes
+    (148 SMs, up to 256 items each), both schemes and the opaque rows."""
+    check_sizes(fp_ctx, oracle, n)
 
 
 def meeting_signatures(oracle):
@@ -220,9 +224,7 @@ def test_meeting_signatures_are_what_they_say(oracle):
     assert not oracle.schnorr_verify_batch(sm, sp, ss).any()
 
 
-@pytest.mark.gpu
-def test_sums_that_meet(fp_ctx, oracle):
-    """Equal and opposite sums among ordinary items."""
+def check_meeting(fp_ctx, oracle):
     em, ep, es, sm, sp, ss = meeting_signatures(oracle)
     om, op, os_ = ecdsa_corpus(oracle, 60, 23)
     em, ep, es = (np.concatenate([a, b])[::-1].copy() for a, b in ((em, om), (ep, op), (es, os_)))
@@ -230,3 +232,31 @@ def test_sums_that_meet(fp_ctx, oracle):
     om, op, os_ = schnorr_corpus(oracle, 60, 24, tamper=0.1)
     sm, sp, ss = (np.concatenate([a, b])[::-1].copy() for a, b in ((sm, om), (sp, op), (ss, os_)))
     assert (fp_ctx.schnorr_verify_batch(sm, sp, ss) == oracle.schnorr_verify_batch(sm, sp, ss)).all()
+
+
+@pytest.mark.gpu
+def test_sums_that_meet(fp_ctx, oracle):
+    """Equal and opposite sums among ordinary items."""
+    check_meeting(fp_ctx, oracle)
+
+
+@pytest.fixture(scope="module")
+def team_ctx():
+    """A context whose calls of every size take the small-call kernel (four warps per 32 signatures)."""
+    import ultrafastsecp256k1_b200 as uf
+    with uf.GpuContext(0) as ctx:
+        for k in (0, 1):
+            ctx.set_lanes(k, 2, 1 << 22)
+        yield ctx
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64, 147 * 32 + 5, 9473])
+def test_team_block_edges(team_ctx, oracle, n):
+    """Part of a block to more blocks than run at once."""
+    check_sizes(team_ctx, oracle, n)
+
+
+@pytest.mark.gpu
+def test_team_sums_that_meet(team_ctx, oracle):
+    check_meeting(team_ctx, oracle)

@@ -49,8 +49,8 @@ int env_int(const char* name, int dflt) {
 cudaError_t Backend::launch_verify(int kind, const uint8_t* m, const uint8_t* p, const uint8_t* s, uint32_t n,
                                    uint8_t* out, int collect, cudaStream_t st, size_t call_items) {
     const int k = kind & 1;
-    if (kind != 2 && call_items <= pair_items_[k])
-        return launch_verify_pair(kind, m, p, s, n, d_gtab_, out, collect, st);
+    if (call_items <= pair_items_[k])
+        return launch_verify_team(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, st);
     const bool small = small_variant_[k] >= 0 && call_items <= small_items_[k];
     if (!small && inv_group_[k] > 1)
         return launch_verify_fp(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, sms_, st);
@@ -367,7 +367,7 @@ int Backend::init(int device_index) {
     for (int v = 0; v < kVerifyVariants; ++v)
         for (int k = 0; k < 2; ++k) grid_[v][k] = std::max(1, kOccupancy[v](k)) * sms_;
     queue_grid_ = std::max(1, verify_queue_occupancy()) * sms_;
-    if ((e = verify_fp_init()) != cudaSuccess) return cuda_error(e, "verify kernel set-up");
+    if ((e = verify_fp_init()) != cudaSuccess || (e = verify_team_init()) != cudaSuccess) return cuda_error(e, "verify kernel set-up");
     queue_pair_grid_ = std::max(1, verify_pair_occupancy()) * sms_;   // also the two-lane kernels' shared-memory opt-in
     load_tuning();
     // generator tables of the window widths the chosen variants use; a variant

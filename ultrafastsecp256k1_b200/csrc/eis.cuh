@@ -99,10 +99,11 @@ UF_HD void fd_beta_pow(Fd& r, uint32_t e) {
 }
 
 // (x, y) times the unit beta^e, sign: x2 strict, y2 negated where neg.
+template <bool kCalls>
 UF_HD void eis_unit(Fd& x, Fd& y, uint32_t e, bool neg) {
     Fd b;
     fd_beta_pow(b, e);
-    x = fd_mul(x, b);
+    x = jf_mul<kCalls>(x, b);
     const double s = neg ? -1.0 : 1.0;
     UF_UNROLL
     for (int i = 0; i < 5; ++i) y.v[i] *= s;
@@ -119,9 +120,11 @@ UF_HD void eis_unit(Fd& x, Fd& y, uint32_t e, bool neg) {
 // pass from the last entry down multiplies the entries up by the later H's
 // (4M + 1S each).  (If an addition meets equal or opposite points, which a point
 // of order n never does, H becomes 0 and everything computed from it too.)
+//
+// eis_path is the first pass (hs[k]: Z of entry k over Z of entry k - 1),
+// eis_scale multiplies one entry by rho = Z of the last entry over its own.
 template <class Tab>
-UF_HDI Fd eis_table(const Tab& tab, const Fd& px, const Fd& py) {
-    Fd hs[kEisTab];              // Z of entry k over Z of entry k - 1
+UF_HDI void eis_path(const Tab& tab, const Fd& px, const Fd& py, Fd hs[kEisTab]) {
     Fd ux = px, uy = py, X = px, Y = py;
     uint32_t cur = 0;            // the unit that U holds
     tab.store(0, X, Y);
@@ -147,22 +150,34 @@ UF_HDI Fd eis_table(const Tab& tab, const Fd& px, const Fd& py) {
         ux = W1;
         tab.store(k, X, Y);
     }
+}
+
+template <class Tab>
+UF_HDI void eis_scale(const Tab& tab, int k, const Fd& rho) {
+    Fd X, Y;
+    const Fd r2 = fdc_sqr(rho);
+    tab.load(k, X, Y);
+    X = fdc_mul(X, r2);
+    Y = fdc_mul(Y, fdc_mul(r2, rho));
+    tab.store(k, X, Y);
+}
+
+template <class Tab>
+UF_HDI Fd eis_table(const Tab& tab, const Fd& px, const Fd& py) {
+    Fd hs[kEisTab];
+    eis_path(tab, px, py, hs);
     Fd rho = hs[kEisTab - 1];
     UF_NOUNROLL
     for (int k = kEisTab - 2; k >= 0; --k) {
-        const Fd r2 = fdc_sqr(rho);
-        tab.load(k, X, Y);
-        X = fdc_mul(X, r2);
-        Y = fdc_mul(Y, fdc_mul(r2, rho));
-        tab.store(k, X, Y);
+        eis_scale(tab, k, rho);
         if (k > 0) rho = fdc_mul(rho, hs[k]);
     }
     return rho;
 }
 
 // One digit of the sum over the table, most significant first: R <- 8 R + digit
-// (129 doublings and at most 44 additions in all).
-template <class Tab>
+// (129 doublings and at most 44 additions in all).  kCalls as in jacd.cuh.
+template <bool kCalls, class Tab>
 UF_HD void eis_add_digit(JacD& R, uint32_t e, bool top, const Tab& tab) {
     if (!top) {
         UF_NOUNROLL
@@ -171,8 +186,8 @@ UF_HD void eis_add_digit(JacD& R, uint32_t e, bool top, const Tab& tab) {
     if (e != kEisZero) {
         Fd x, y;
         tab.load((int)(e & 15u), x, y);
-        eis_unit(x, y, (e >> 4) & 3u, (e & 64u) != 0);
-        R = jacd_add_aff_c(R, x, y);
+        eis_unit<kCalls>(x, y, (e >> 4) & 3u, (e & 64u) != 0);
+        R = jacd_add_aff_t<kCalls>(R, x, y);
     }
 }
 
@@ -181,7 +196,7 @@ UF_HD JacD eis_mul(const uint8_t* dig, const Tab& tab) {
     JacD R;
     jacd_set_inf(R);
     UF_NOUNROLL
-    for (int i = kEisDigits - 1; i >= 0; --i) eis_add_digit(R, dig[i], i == kEisDigits - 1, tab);
+    for (int i = kEisDigits - 1; i >= 0; --i) eis_add_digit<false>(R, dig[i], i == kEisDigits - 1, tab);
     return R;
 }
 

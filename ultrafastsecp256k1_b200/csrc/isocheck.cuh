@@ -35,7 +35,10 @@ constexpr size_t kCombBytes = (size_t)kCombWindows * kCombTab * 64;
 
 #if defined(__CUDACC__)
 
-__device__ __forceinline__ JacD comb_mul(Sc s, const uint4* __restrict__ comb) {
+// Windows [first, last) of s G (all of them: 0, kCombWindows).  kCalls as in jacd.cuh.
+template <bool kCalls>
+__device__ __forceinline__ JacD comb_mul(Sc s, const uint4* __restrict__ comb, int first = 0,
+                                         int last = kCombWindows) {
     JacD B;
     Sc k = s;
     const bool flip = !sc_is_low(s.v);         // |k| < 2^255: the last window takes no carry out
@@ -43,14 +46,14 @@ __device__ __forceinline__ JacD comb_mul(Sc s, const uint4* __restrict__ comb) {
     jacd_set_inf(B);
     uint32_t carry = 0;
     UF_NOUNROLL
-    for (int i = 0; i < kCombWindows; ++i) {
+    for (int i = 0; i < last; ++i) {
         const uint32_t w = (k.v[0] & 0xFFFFu) + carry;
         carry = w > (uint32_t)kCombTab ? 1u : 0u;
         const int d = (int)w - (int)(carry << 16);
         UF_UNROLL
         for (int j = 0; j < 7; ++j) k.v[j] = (k.v[j] >> 16) | (k.v[j + 1] << 16);
         k.v[7] >>= 16;
-        if (d != 0) {
+        if (d != 0 && i >= first) {
             const uint4* q = comb + 4 * ((size_t)i * kCombTab + (size_t)((d < 0 ? -d : d) - 1));
             const uint4 x0 = __ldg(q), x1 = __ldg(q + 1), y0 = __ldg(q + 2), y1 = __ldg(q + 3);
             const uint32_t xw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
@@ -61,7 +64,7 @@ __device__ __forceinline__ JacD comb_mul(Sc s, const uint4* __restrict__ comb) {
             const double sg = (d < 0) != flip ? -1.0 : 1.0;
             UF_UNROLL
             for (int j = 0; j < 5; ++j) y.v[j] *= sg;
-            B = jacd_add_aff(B, x, y);
+            B = kCalls ? jacd_add_aff_t<true>(B, x, y) : jacd_add_aff(B, x, y);
         }
     }
     return B;

@@ -83,6 +83,10 @@ cudaError_t launch_verify_fp(int kind, const uint8_t* msgs, const uint8_t* pubs,
                              const void* d_gtab, const void* d_comb, uint8_t* out, int collect, int sms,
                              cudaStream_t s);
 cudaError_t verify_fp_init();
+// Small calls: four warps per 32 signatures (kernels_team.cu).
+cudaError_t launch_verify_team(int kind, const uint8_t* msgs, const uint8_t* pubs, const uint8_t* sigs, uint32_t n,
+                               const void* d_gtab, const void* d_comb, uint8_t* out, int collect, cudaStream_t s);
+cudaError_t verify_team_init();
 // Fills the generator window table (comb_table_bytes() bytes; isocheck.cuh).
 size_t comb_table_bytes();
 cudaError_t launch_comb_init(void* d_comb, cudaStream_t s);
@@ -162,11 +166,8 @@ int verify_queue_occupancy();
 // for the build pass.
 cudaError_t launch_key_passes(const QueueArgs& a, int grid, cudaStream_t s);
 
-// Two lanes per signature (kernels_pair.cu), kind 0 ECDSA (compact) or 1
-// BIP-340, for small calls; verify_pair_occupancy() also opts the kernels in
-// to their shared memory (call once per device).
-cudaError_t launch_verify_pair(int kind, const uint8_t* msgs, const uint8_t* pubs, const uint8_t* sigs, uint32_t n,
-                               const void* d_gtab, uint8_t* out, int collect, cudaStream_t s);
+// Two lanes per signature (kernels_pair.cu): resident blocks per SM of the
+// queue form below; also opts it in to its shared memory (call once per device).
 int verify_pair_occupancy();
 // The work-queue form of the two-lane kernels (no key cache), same contract as
 // launch_verify_queue; `grid` from verify_pair_occupancy().

@@ -1,7 +1,7 @@
-// Two lanes per signature, for small calls.
+// Two lanes per signature, for small mixed-job launches.
 //
 // No reference counterpart (the reference verifies one signature per
-// thread).  A call of a few thousand signatures occupies a few warps per SM,
+// thread).  A launch of a few thousand signatures occupies a few warps per SM,
 // so its time is one thread's verify latency, not the device's throughput.
 // Here lanes 2t and 2t+1 verify signature t together: both parse the
 // signature, decompress the key, compute the scalars and build the 1P..8P
@@ -129,31 +129,6 @@ __device__ __forceinline__ bool pair_item(const uint8_t* msg, const uint8_t* pub
     return ok;
 }
 
-// Two threads per item; the grid covers 2n threads exactly (no grid-stride
-// loop, so every lane of a warp reaches the shuffles once).
-template <int kKind>
-__global__ void __launch_bounds__(kPairThreads)
-k_verify_pair(const uint8_t* __restrict__ msgs, const uint8_t* __restrict__ pubs, const uint8_t* __restrict__ sigs,
-              uint32_t n, const uint4* __restrict__ gt, uint8_t* __restrict__ out, int collect) {
-    extern __shared__ uint4 smem_tab[];
-    const SmemTab tab{smem_tab + threadIdx.x, blockDim.x};
-    const GlobalGT g{gt};
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t i = tid >> 1;
-    const int half = (int)(tid & 1u);
-    const bool valid = i < n;
-    const uint32_t j = valid ? i : 0;      // an in-bounds index for the (unused) pointers
-    const bool ok = pair_item<kKind>(msgs + 32ull * j, pubs + (kKind == 0 ? 33ull : 32ull) * j, sigs + 64ull * j,
-                                     valid, half, tab, g, NoPubCache());
-    if (valid && half == 0) {
-        if (collect) {
-            if (ok) out[i] = 0;
-        } else {
-            out[i] = ok ? 1 : 0;
-        }
-    }
-}
-
 // The work-queue form (the per-kind queues of kernels_queue.cu): each warp
 // claims 16 items and verifies them with its 16 lane pairs, until its queue is
 // empty.  The claim is warp-uniform, so every lane reaches the shuffles of each
@@ -189,20 +164,6 @@ k_verify_queue_pair(QueueArgs a, const uint4* __restrict__ gt, unsigned int* __r
 
 }  // namespace
 
-cudaError_t launch_verify_pair(int kind, const uint8_t* msgs, const uint8_t* pubs, const uint8_t* sigs, uint32_t n,
-                               const void* d_gtab, uint8_t* out, int collect, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    const size_t smem = kPairThreads * kVerifySmemPerThread;
-    const uint64_t threads = 2ull * n;
-    const int grid = (int)((threads + kPairThreads - 1) / kPairThreads);
-    const uint4* gt = reinterpret_cast<const uint4*>(d_gtab);
-    if (kind == 0)
-        k_verify_pair<0><<<grid, kPairThreads, smem, s>>>(msgs, pubs, sigs, n, gt, out, collect);
-    else
-        k_verify_pair<1><<<grid, kPairThreads, smem, s>>>(msgs, pubs, sigs, n, gt, out, collect);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_verify_queue_pair(const QueueArgs& a, const void* d_gtab, unsigned int* d_head, int grid,
                                      cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join) {
     const size_t smem = kPairThreads * kVerifySmemPerThread;
@@ -237,8 +198,6 @@ int verify_pair_occupancy() {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, f, kPairThreads, smem);
         lo = blocks < lo ? blocks : lo;
     };
-    probe(k_verify_pair<0>);
-    probe(k_verify_pair<1>);
     probe(k_verify_queue_pair<0>);
     probe(k_verify_queue_pair<1>);
     return lo;

@@ -23,52 +23,12 @@
 #include "verify.cuh"
 #include "dev_tables.cuh"
 #include "isocheck.cuh"
+#include "verify_fp.cuh"
 
 namespace uf {
 namespace {
 
 constexpr int kFpThreads = 256;
-constexpr size_t kFpSmemPerThread = (size_t)kEisTab * 80;
-
-// A thread's 11-point table: [entry][5 pairs of doubles][thread], so that a
-// thread's reads stay in its own 16-byte column (no bank conflict whatever the
-// lanes' digits are).
-struct EisTab {
-    double2* base;
-    uint32_t stride;
-    __device__ __forceinline__ void store(int k, const Fd& x, const Fd& y) const {
-        double2* p = base + (uint32_t)(k * 5) * stride;
-        p[0] = make_double2(x.v[0], x.v[1]);
-        p[stride] = make_double2(x.v[2], x.v[3]);
-        p[2 * stride] = make_double2(x.v[4], y.v[0]);
-        p[3 * stride] = make_double2(y.v[1], y.v[2]);
-        p[4 * stride] = make_double2(y.v[3], y.v[4]);
-    }
-    __device__ __forceinline__ void load(int k, Fd& x, Fd& y) const {
-        const double2* p = base + (uint32_t)(k * 5) * stride;
-        const double2 a = p[0], b = p[stride], c = p[2 * stride], d = p[3 * stride], e = p[4 * stride];
-        x.v[0] = a.x; x.v[1] = a.y; x.v[2] = b.x; x.v[3] = b.y; x.v[4] = c.x;
-        y.v[0] = c.y; y.v[1] = d.x; y.v[2] = d.y; y.v[3] = e.x; y.v[4] = e.y;
-    }
-};
-
-// One item by the plain per-thread verification (rare): its 512-byte table lies
-// in the thread's own column of the same shared memory.
-template <int kKind>
-__device__ __noinline__ bool plain_verify(const uint8_t* msgs, const uint8_t* pubs, const uint8_t* sigs, uint32_t i,
-                                          const uint4* gt, uint4* smem) {
-    SmemTab tab{smem + threadIdx.x, blockDim.x};
-    const GlobalGT g{gt};
-    uint32_t mw[8], sw[16];
-    load_words8(mw, msgs + 32ull * i);
-    load_words8(sw, sigs + 64ull * i);
-    load_words8(sw + 8, sigs + 64ull * i + 32);
-    if (kKind == 0) return ecdsa_verify_one(mw, pubs + 33ull * i, sw, tab, g);
-    if (kKind == 2) return ecdsa_verify_opaque_one(mw, pubs + 33ull * i, sw, tab, g);
-    uint32_t pw[8];
-    load_words8(pw, pubs + 32ull * i);
-    return schnorr_verify_one(mw, pw, sw, tab, g);
-}
 
 // kKind: 0 ECDSA (compact r || s, low-S), 1 BIP-340, 2 ECDSA (opaque
 // little-endian r, s; high-S normalised).
@@ -82,74 +42,15 @@ k_verify_fp(const uint8_t* __restrict__ msgs, const uint8_t* __restrict__ pubs, 
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool ok = i < n, odd = false;
     uint32_t px[8], r[8];
-    Sc s, b;             // R = s G + b P
+    Sc a, b;             // R = a G + b P
     uint8_t dig[kEisDigits];
-    if (kKind == 1) {
-        // BIP-340: parse and challenge (schnorr_verify_one)
-        if (ok) {
-            uint32_t mw[8], sw[16], pw[8];
-            load_words8(mw, msgs + 32ull * i);
-            load_words8(sw, sigs + 64ull * i);
-            load_words8(sw + 8, sigs + 64ull * i + 32);
-            load_words8(pw, pubs + 32ull * i);
-            words_be_to_limbs(r, sw);
-            words_be_to_limbs(s.v, sw + 8);
-            words_be_to_limbs(px, pw);
-            ok = limbs_lt_p(r) && !sc_is_zero(s) && limbs_lt_n(s.v) && limbs_lt_p(px);
-            uint32_t rbe[8], pbe[8], mbe[8], h[8];
-            UF_UNROLL
-            for (int k = 0; k < 8; ++k) {
-                rbe[k] = bswap32(sw[k]);
-                pbe[k] = bswap32(pw[k]);
-                mbe[k] = bswap32(mw[k]);
-            }
-            bip340_challenge(h, rbe, pbe, mbe);
-            Sc e;
-            UF_UNROLL
-            for (int k = 0; k < 8; ++k) e.v[k] = h[7 - k];
-            sc_reduce_once(e);
-            sc_neg(b, e);
-        }
-    } else {
-        // ECDSA: parse, u1 and u2
-        if (ok) {
-            uint32_t sw[16];
-            load_words8(sw, sigs + 64ull * i);
-            load_words8(sw + 8, sigs + 64ull * i + 32);
-            if (kKind == 0) {
-                words_be_to_limbs(r, sw);
-                words_be_to_limbs(s.v, sw + 8);
-            } else {
-                UF_UNROLL
-                for (int k = 0; k < 8; ++k) {
-                    r[k] = sw[k];
-                    s.v[k] = sw[8 + k];
-                }
-            }
-            ok = !is_zero256(r) && limbs_lt_n(r) && !sc_is_zero(s) && limbs_lt_n(s.v);
-            if (ok) {
-                if (kKind == 0) ok = sc_is_low(s.v);
-                else if (!sc_is_low(s.v)) sc_neg(s, s);
-            }
-            const uint8_t* pub = pubs + 33ull * i;
-            const uint8_t prefix = pub[0];
-            odd = prefix == 0x03;
-            be32_to_limbs(px, pub + 1);
-            ok = ok && (prefix == 0x02 || prefix == 0x03) && limbs_lt_p(px);
-        }
-        if (ok) {
-            uint32_t mw[8];
-            load_words8(mw, msgs + 32ull * i);
-            Sc z, rs;
-            words_be_to_limbs(z.v, mw);
-            sc_reduce_once(z);
-            UF_UNROLL
-            for (int k = 0; k < 8; ++k) rs.v[k] = r[k];
-            Sc w;
-            sc_inv(w, s);
-            sc_mul(s, z, w);
-            sc_mul(b, rs, w);
-        }
+    const uint8_t* msg = msgs + 32ull * i;
+    const uint8_t* pub = pubs + (kKind == 1 ? 32ull : 33ull) * i;
+    const uint8_t* sig = sigs + 64ull * i;
+    if (ok) {
+        Sc s;
+        ok = fp_parse_sig<kKind>(r, s, sig) && fp_parse_key<kKind>(px, odd, pub);
+        if (ok) fp_scalars<kKind>(a, b, r, s, msg, pub, sig);
     }
     Fd c, den, zc;
     JacD A;
@@ -167,21 +68,21 @@ k_verify_fp(const uint8_t* __restrict__ msgs, const uint8_t* __restrict__ pubs, 
     __syncthreads();
     UF_NOUNROLL
     for (int q = kEisDigits - 1; q >= 0; --q) {
-        if (ok) eis_add_digit(A, dig[q], q == kEisDigits - 1, tab);
+        if (ok) eis_add_digit<false>(A, dig[q], q == kEisDigits - 1, tab);
     }
     __syncthreads();
     if (ok) {
         A.Z = fdc_mul(A.Z, zc);
         if (kKind == 1) {
+            // the scalar and r again from the signature: not held over the main loop
             uint32_t sw[8];
-            load_words8(sw, sigs + 64ull * i + 32);
-            words_be_to_limbs(s.v, sw);
+            load_words8(sw, sig + 32);
+            words_be_to_limbs(a.v, sw);
         }
-        const JacD B = comb_mul(s, comb);
+        const JacD B = comb_mul<false>(a, comb);
         if (kKind == 1) {
-            // s went into B; r from the signature again
             uint32_t sw[8];
-            load_words8(sw, sigs + 64ull * i);
+            load_words8(sw, sig);
             words_be_to_limbs(r, sw);
         }
         plain = !iso_prepare<kKind == 1>(tab, den, A, B, c, r);
@@ -199,7 +100,7 @@ k_verify_fp(const uint8_t* __restrict__ msgs, const uint8_t* __restrict__ pubs, 
             if (kKind != 1 && !ok && r_below_p_minus_n(r)) ok = plain = true;
         }
     }
-    if (ok && plain) ok = plain_verify<kKind>(msgs, pubs, sigs, i, gt, smem);
+    if (ok && plain) ok = plain_verify<kKind>(msg, pub, sig, gt, smem + threadIdx.x, blockDim.x);
     if (i < n) {
         if (collect) {
             if (ok) out[i] = 0;
