@@ -102,9 +102,9 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_inject_fault(ufsecp_gpu_ctx* ctx, uint3
  * slot and a build pass fills the new slots, so the verify warps never mix
  * lanes that build a table with lanes that copy one.  Verdicts never depend on
  * the table.  log2_slots: 0 = off; 8..24 = an empty table of 2^log2_slots
- * slots of 576 bytes (a table of that size is emptied in place, another size
+ * slots of 768 bytes (a table of that size is emptied in place, another size
  * is made on the next verify_jobs call).  Default: 18
- * (151 MB), from the tuning file's key_table_log2 or the environment
+ * (201 MB), from the tuning file's key_table_log2 or the environment
  * variable UFSECP_B200_KEY_TABLE when set.  Slots are never evicted: when a
  * key's probe window is full it is verified without the table.
  * key_table_stats: out[0] lookups (items whose key parsed) and out[1] hits
@@ -245,7 +245,7 @@ typedef struct {
     uint32_t max_launch_items;      /* 1..65536 */
     uint64_t memory_budget_bytes;
     uint32_t batch_window_us;       /* 0: launch as soon as a slot is free */
-    uint32_t key_cache_log2;        /* resident key table of 2^k slots, 576 B each:
+    uint32_t key_cache_log2;        /* resident key table of 2^k slots, 768 B each:
                                        0 or 1 = none, else 8..24 (NULL config: 18) */
 } ufsecp_gpu_ext_server_config_t;
 typedef struct {

@@ -64,9 +64,6 @@ _WINDOW_FLAGS = [
 VARIANTS = {"kernels_verify.cu": _VARIANT_FLAGS + _WINDOW_FLAGS, "kernels_probe.cu": _VARIANT_FLAGS,
             "kernels_queue.cu": [("", _BEST_FLAGS)], "kernels_noalloc.cu": [("", _BEST_FLAGS)],
             "kernels_verify_fp.cu": [("", _BEST_FLAGS)], "kernels_team.cu": [("", _BEST_FLAGS)],
-            # small calls are latency-bound: the two-lane kernel takes variant 6's
-            # code generation (field ops inlined into out-of-line point ops)
-            "kernels_pair.cu": [("", ["-DUF_NOINLINE_POINT", "-DUF_PTX_MUL"])],
             "rlc.cu": [("", _BEST_FLAGS)], "kernels_ops.cu": [("", _BEST_FLAGS)],
             # the RLC kernels with one serial chain per segment or window run few
             # threads: field and point operations inlined, for overlap inside a chain

@@ -366,9 +366,9 @@ int Backend::init(int device_index) {
     if ((e = cudaStreamSynchronize(stream_)) != cudaSuccess) return cuda_error(e, "gtable init");
     for (int v = 0; v < kVerifyVariants; ++v)
         for (int k = 0; k < 2; ++k) grid_[v][k] = std::max(1, kOccupancy[v](k)) * sms_;
-    queue_grid_ = std::max(1, verify_queue_occupancy()) * sms_;
-    if ((e = verify_fp_init()) != cudaSuccess || (e = verify_team_init()) != cudaSuccess) return cuda_error(e, "verify kernel set-up");
-    queue_pair_grid_ = std::max(1, verify_pair_occupancy()) * sms_;   // also the two-lane kernels' shared-memory opt-in
+    if ((e = verify_fp_init()) != cudaSuccess || (e = verify_team_init()) != cudaSuccess ||
+        (e = verify_queue_init()) != cudaSuccess)
+        return cuda_error(e, "verify kernel set-up");
     load_tuning();
     // generator tables of the window widths the chosen variants use; a variant
     // whose tables cannot be made falls back to variant 4
@@ -691,11 +691,9 @@ int Backend::verify_queue_jobs(const VerifyJob* jobs, size_t n_jobs) {
         }
         part[q].clear();
         // the first sub-calls ramp up from kPipeFirst items, so the device
-        // starts while the CPU packs the next one, to one wave of the queue
-        // kernel's resident grid (56,832 items on a 148-SM B200): a sub-call
-        // of 65,536 items was 1.15 waves and ran its tail alone (mixed jobs in
-        // one call 28.8 -> 30.0 M sigs/s, one BIP-340 job 32.2 -> 33.7 M)
-        const size_t wave = std::max<size_t>(kPipeFirst, std::min(kJobsPipeItems, (size_t)queue_grid_ * kVerifyThreads));
+        // starts while the CPU packs the next one, to one wave of the verify
+        // kernel's full blocks (256 items per SM: 37,888 on a 148-SM B200)
+        const size_t wave = std::max<size_t>(kPipeFirst, std::min(kJobsPipeItems, (size_t)sms_ * 256));
         const size_t cap = std::min(wave, kPipeFirst << std::min(k, 8));
         size_t n = 0;
         while (j < n_jobs && n < cap) {

@@ -62,6 +62,7 @@ public:
     int device() const { return dev_; }
     cudaStream_t stream() const { return stream_; }
     const void* gtab() const { return d_gtab_; }
+    const void* comb() const { return d_comb_; }
     int sms() const { return sms_; }
 
     // Host buffers in, host verdicts out; synchronous (the reference contract).
@@ -120,10 +121,8 @@ public:
     // tuning file's rlc_affine or UFSECP_B200_RLC_AFFINE may turn it off.
     bool rlc_affine() const { return rlc_affine_; }
     void set_rlc_affine(bool on) { rlc_affine_ = on; }
-    int queue_grid() const { return queue_grid_; }
-    int queue_pair_grid() const { return queue_pair_grid_; }
     // Mixed-job launches of at most this many items (both kinds together) run
-    // the two-lane queue kernels: the smaller of the kinds' two-lane limits.
+    // four warps per 32 signatures: the smaller of the kinds' limits.
     uint32_t queue_pair_items() const { return std::min(pair_items_[0], pair_items_[1]); }
     // Per-item batch operations (ops.cpp): host buffers, synchronous.
     int xonly_validate(const uint8_t* keys32, size_t n, uint8_t* out);
@@ -220,8 +219,6 @@ private:
     // large device-buffer calls: second stream with fork / join events
     cudaStream_t dstream_ = nullptr;
     cudaEvent_t dfork_ = nullptr, djoin_ = nullptr;
-    int queue_grid_ = 0;
-    int queue_pair_grid_ = 0;
     std::unique_ptr<BatchSlot> batch_[2];   // slots of the synchronous mixed-batch call (two for large calls)
     std::unique_ptr<KeyTable> keys_;        // resident key table of verify_jobs (made on first use)
     int verify_queue_jobs(const VerifyJob* jobs, size_t n_jobs);   // kinds 0 and 1

@@ -49,11 +49,13 @@ BatchSlot::~BatchSlot() {
     for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
     graphs_.clear();
     if (stream2_) cudaStreamSynchronize(stream2_);
+    if (stream3_) cudaStreamSynchronize(stream3_);
     if (done_) cudaEventDestroy(done_);
     if (fork_) cudaEventDestroy(fork_);
     if (join_) cudaEventDestroy(join_);
+    if (join3_) cudaEventDestroy(join3_);
     if (stream2_) cudaStreamDestroy(stream2_);
-    if (d_head_) cudaFree(d_head_);
+    if (stream3_) cudaStreamDestroy(stream3_);
     pinned_.release();
     big_pinned_.release();
     dev_.release();
@@ -68,9 +70,10 @@ int BatchSlot::init(Backend* be, bool use_graphs) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream2_, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream3_, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join_, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join3_, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done_, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMalloc(&d_head_, 256);
     if (e == cudaSuccess && use_graphs) {
         // the graph buckets all bind this one staging pair, sized for the largest bucket
         const QueueLayout maxl(kGraphMaxItems, kGraphMaxItems);
@@ -81,15 +84,15 @@ int BatchSlot::init(Backend* be, bool use_graphs) {
     return kOk;
 }
 
-// Small layouts run two lanes per signature (the backend's tuned limit); the
+// Small layouts run four warps per 32 signatures (the backend's tuned limit); the
 // choice is part of the graph key, so a changed limit never replays a graph
 // captured with the other kernels.
-bool BatchSlot::two_lanes(const QueueArgs& a) const {
+bool BatchSlot::small_launch(const QueueArgs& a) const {
     return (uint64_t)a.cap_e + a.cap_s <= be_->queue_pair_items();
 }
 
 uint64_t BatchSlot::graph_key(const QueueArgs& a) const {
-    return ((uint64_t)a.cap_e << 32) | a.cap_s | (two_lanes(a) ? (1ull << 63) : 0);
+    return ((uint64_t)a.cap_e << 32) | a.cap_s | (small_launch(a) ? (1ull << 63) : 0);
 }
 
 QueueArgs BatchSlot::args_for(uint8_t* d) const {
@@ -122,10 +125,8 @@ int BatchSlot::run_direct(const QueueArgs& a) {
     uint8_t* d = staged_big_ ? (uint8_t*)big_dev_.p : (uint8_t*)dev_.p;
     cudaError_t e = cudaMemcpyAsync(d, h, layout_.in_bytes, cudaMemcpyHostToDevice, stream_);
     if (e == cudaSuccess)
-        e = two_lanes(a) ? launch_verify_queue_pair(a, be_->gtab(), d_head_, be_->queue_pair_grid(), stream_, stream2_,
-                                                    fork_, join_)
-                         : launch_verify_queue(a, be_->gtab(), d_head_, be_->queue_grid(), stream_, stream2_, fork_,
-                                               join_);
+        e = launch_verify_queue(a, small_launch(a), be_->gtab(), be_->comb(), be_->sms(),
+                                QueueStreams{stream_, stream2_, stream3_, fork_, join_, join3_});
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h + layout_.e_out, d + layout_.e_out, layout_.out_bytes, cudaMemcpyDeviceToHost, stream_);
     if (e != cudaSuccess) return be_->cuda_error(e, "batch enqueue");

@@ -5,8 +5,8 @@
 // src/gpu/src/gpu_backend_cuda.cu:972-1028).  A BatchSlot owns one stream, a
 // pinned host staging buffer and its device twin laid out as QueueLayout
 // (kernels.h).  enqueue() packs any number of caller jobs into the staging
-// buffer, then issues  H2D copy -> queue-head reset -> persistent queue kernel
-// -> D2H copy  on the slot's stream.  For staging layouts up to
+// buffer, then issues  H2D copy -> key passes -> verify kernels -> D2H copy  on
+// the slot's stream.  For staging layouts up to
 // kGraphMaxItems per kind the sequence is a CUDA graph captured once per
 // capacity bucket (powers of two from 256) and replayed; the kernel reads the
 // live item counts from the copied header, so a bucket's graph serves every
@@ -72,7 +72,7 @@ public:
 
 private:
     int run_direct(const QueueArgs& a);
-    bool two_lanes(const QueueArgs& a) const;
+    bool small_launch(const QueueArgs& a) const;
     uint64_t graph_key(const QueueArgs& a) const;
     int run_graph(const QueueArgs& a, uint64_t key);
     QueueArgs args_for(uint8_t* dev_base) const;
@@ -81,9 +81,9 @@ private:
     bool use_graphs_ = true;
     cudaStream_t stream_ = nullptr;
     cudaStream_t stream2_ = nullptr;           // the BIP-340 queue's branch
-    cudaEvent_t fork_ = nullptr, join_ = nullptr;
+    cudaStream_t stream3_ = nullptr;           // the key passes' branch of small launches
+    cudaEvent_t fork_ = nullptr, join_ = nullptr, join3_ = nullptr;
     cudaEvent_t done_ = nullptr;
-    unsigned int* d_head_ = nullptr;
     HostBuf pinned_;                 // graph-bucket staging (fixed size, graphs bind it)
     DevBuf dev_;
     HostBuf big_pinned_;             // direct-path staging (grows)

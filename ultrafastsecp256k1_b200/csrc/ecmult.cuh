@@ -20,7 +20,6 @@
 #include "fe.cuh"
 #include "fn.cuh"
 #include "point.cuh"
-#include "pubcache.cuh"
 
 namespace uf {
 
@@ -135,13 +134,11 @@ UF_HD void add_gtab(Jac& R, const GT& gt, int d, bool sneg, int lam) {
     jac_add_aff(R, x, y);
 }
 
-// R = a*G + b*P for P = (px, py) on the curve (not infinity).  With
-// have_tab the caller already filled `tab` (a resident key) and px, py are not
-// read; otherwise the table is built here, after the digit recoding (the order
-// that keeps the kernel at 3 blocks per SM).
+// R = a*G + b*P for P = (px, py) on the curve (not infinity).  The table is
+// built after the digit recoding (the order that keeps the kernel at 3 blocks
+// per SM).
 template <class Tab, class GT>
-UF_HDI void dual_mul_c(Jac& R, const Sc& a, const Fe& px, const Fe& py, const Sc& b, Tab& tab, const GT& gt,
-                       bool have_tab) {
+UF_HDI void dual_mul(Jac& R, const Sc& a, const Fe& px, const Fe& py, const Sc& b, Tab& tab, const GT& gt) {
     GlvSplit sa, sb;
     glv_split(sa, a);
     glv_split(sb, b);
@@ -151,7 +148,7 @@ UF_HDI void dual_mul_c(Jac& R, const Sc& a, const Fe& px, const Fe& py, const Sc
     booth_recode<kWP, kNWP>(dp2, sb.k2);
     booth_recode<kWG, kNWG>(dg1, sa.k1);
     booth_recode<kWG, kNWG>(dg2, sa.k2);
-    if (!have_tab) build_ptable(tab, px, py);
+    build_ptable(tab, px, py);
     Fe beta;
     fe_beta(beta);
     jac_set_inf(R);
@@ -165,46 +162,6 @@ UF_HDI void dual_mul_c(Jac& R, const Sc& a, const Fe& px, const Fe& py, const Sc
             add_gtab(R, gt, dg2[i / kGEvery], sa.neg2, 1);
         }
     }
-}
-
-// One lane's half of R = a*G + b*P when two lanes share a signature: half 0
-// sums the a1*G and b1*P streams, half 1 the a2*(lambda G) and b2*(lambda P)
-// streams (the GLV halves), each with the full 128 doublings, so that the two
-// partial sums add up to R.  Both lanes build the same P table in their own
-// shared-memory slots (the same instruction stream, so no divergence), unless
-// have_tab says the caller already filled `tab`.
-template <class Tab, class GT>
-UF_HDI void dual_mul_half(Jac& R, const Sc& a, const Fe& px, const Fe& py, const Sc& b, Tab& tab, const GT& gt,
-                          int half, bool have_tab = false) {
-    GlvSplit sa, sb;
-    glv_split(sa, a);
-    glv_split(sb, b);
-    uint32_t kp[4], kg[4];
-    UF_UNROLL
-    for (int i = 0; i < 4; ++i) {
-        kp[i] = half ? sb.k2[i] : sb.k1[i];
-        kg[i] = half ? sa.k2[i] : sa.k1[i];
-    }
-    const bool negp = half ? sb.neg2 : sb.neg1, negg = half ? sa.neg2 : sa.neg1;
-    int8_t dp[kNWP];
-    GDigit dg[kNWG];
-    booth_recode<kWP, kNWP>(dp, kp);
-    booth_recode<kWG, kNWG>(dg, kg);
-    if (!have_tab) build_ptable(tab, px, py);
-    Fe beta;
-    fe_beta(beta);
-    jac_set_inf(R);
-    UF_NOUNROLL
-    for (int i = kNWP - 1; i >= 0; --i) {
-        if (i != kNWP - 1) jac_dbl_n(R, kWP);
-        add_ptab(R, tab, dp[i], negp, half != 0, beta);
-        if (i % kGEvery == 0) add_gtab(R, gt, dg[i / kGEvery], negg, half);
-    }
-}
-
-template <class Tab, class GT>
-UF_HDI void dual_mul(Jac& R, const Sc& a, const Fe& px, const Fe& py, const Sc& b, Tab& tab, const GT& gt) {
-    dual_mul_c(R, a, px, py, b, tab, gt, false);
 }
 
 }  // namespace uf

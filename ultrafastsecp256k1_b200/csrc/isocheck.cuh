@@ -89,6 +89,10 @@ __device__ __forceinline__ void iso_key(Fd& kx, Fd& ky, Fd& c, const uint32_t x[
 //   slots 0: m, g1   1: p1, g2   2: p2, p3   3: p4, c
 // y = m / g1 and y_R = ((p1 - y p2) p3 - p4) / g2, p3 kept negated.
 //
+// A key whose table is known in affine coordinates on secp256k1 itself (the
+// resident key table) goes through the same check with c = 1: its scale is one,
+// so the equation holds exactly when y comes out as 1.
+//
 // iso_prepare returns false for A, B infinite or x_A = x_B; den = g1, for
 // BIP-340 g1 g2.
 template <bool kSchnorr, class Tab>
@@ -126,9 +130,10 @@ __device__ __forceinline__ bool iso_prepare(const Tab& tab, Fd& den, const JacD&
     return true;
 }
 
-// Second half, with inv = 1 / den (canonical limbs).
+// Second half, with inv = 1 / den (canonical limbs).  unit: the key was given on
+// secp256k1 (c = 1).
 template <bool kSchnorr, class Tab>
-__device__ __forceinline__ bool iso_finish(const Tab& tab, const Fe& inv, bool odd) {
+__device__ __forceinline__ bool iso_finish(const Tab& tab, const Fe& inv, bool odd, bool unit = false) {
     Fd fi, m, g1, p1, g2, p4, c;
     fd_unpack(fi, inv.v);
     fd_strict(fi);
@@ -139,7 +144,7 @@ __device__ __forceinline__ bool iso_finish(const Tab& tab, const Fe& inv, bool o
     if (!fd_is_zero(fdc_mul_sub(y, y, c))) return false;
     uint32_t w[8];
     fd_pack(w, y);
-    if (((w[0] & 1u) != 0) != odd) return false;
+    if (((w[0] & 1u) != 0) != (odd || unit)) return false;       // of +-1, 1 is the odd one
     if (kSchnorr) {
         Fd p2, p3;
         tab.load(2, p2, p3);

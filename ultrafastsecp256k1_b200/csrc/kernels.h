@@ -150,29 +150,24 @@ struct QueueArgs {
     unsigned long long* cache_stats = nullptr;
     uint32_t *e_slot = nullptr, *s_slot = nullptr, *todo = nullptr, *todo_count = nullptr;
 };
-constexpr size_t kPubCacheSlotBytes = 576;
+constexpr size_t kPubCacheSlotBytes = 768;
 
-// Zeroes the two queue heads (d_head[0] ECDSA, d_head[1] BIP-340), then
-// launches the per-kind persistent queue kernels (`grid` resident blocks
-// each) over the items described by `a`: kinds with capacity 0 are skipped;
-// with both kinds, the BIP-340 kernel runs on s2 between a fork event recorded
-// on s and a join event s waits for (kernels_queue.cu).  With a key table
-// (a.cache) the resolve and build passes (pubcache.cuh) run first, on s.
-cudaError_t launch_verify_queue(const QueueArgs& a, const void* d_gtab, unsigned int* d_head, int grid,
-                                cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join);
-int verify_queue_occupancy();
-// The key table's resolve and build passes alone (launch_verify_queue and
-// launch_verify_queue_pair call it when a.cache is set); `grid` resident blocks
-// for the build pass.
-cudaError_t launch_key_passes(const QueueArgs& a, int grid, cudaStream_t s);
+// A batch slot's streams: the launch's own, the BIP-340 branch, the key passes'
+// branch of small launches; events for the fork and the two joins.
+struct QueueStreams {
+    cudaStream_t main, second, third;
+    cudaEvent_t fork, join, join3;
+};
 
-// Two lanes per signature (kernels_pair.cu): resident blocks per SM of the
-// queue form below; also opts it in to its shared memory (call once per device).
-int verify_pair_occupancy();
-// The work-queue form of the two-lane kernels (no key cache), same contract as
-// launch_verify_queue; `grid` from verify_pair_occupancy().
-cudaError_t launch_verify_queue_pair(const QueueArgs& a, const void* d_gtab, unsigned int* d_head, int grid,
-                                     cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join);
+// Launches the verify kernels over the items described by `a` (kernels_queue.cu):
+// kinds with capacity 0 are skipped; with both kinds, the BIP-340 kernel runs on
+// its own branch.  team: four warps per 32 signatures (small launches).  With a
+// key table (a.cache) the resolve and build passes (pubcache.cuh) run first, for
+// team launches beside the verify kernels.  verify_queue_init opts the kernels in
+// to their shared memory (once per device).
+cudaError_t launch_verify_queue(const QueueArgs& a, bool team, const void* d_gtab, const void* d_comb, int sms,
+                                const QueueStreams& q);
+cudaError_t verify_queue_init();
 
 // Allocation-free mixed verification (kernels_noalloc.cu): the jobs' buffers
 // are device-accessible memory the caller owns; the queue head and the job

@@ -38,69 +38,9 @@ k_verify_fp(const uint8_t* __restrict__ msgs, const uint8_t* __restrict__ pubs, 
              uint32_t n, const uint4* __restrict__ gt, const uint4* __restrict__ comb, uint8_t* __restrict__ out,
              int collect) {
     extern __shared__ uint4 smem[];
-    const EisTab tab{reinterpret_cast<double2*>(smem) + threadIdx.x, blockDim.x};
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool ok = i < n, odd = false;
-    uint32_t px[8], r[8];
-    Sc a, b;             // R = a G + b P
-    uint8_t dig[kEisDigits];
-    const uint8_t* msg = msgs + 32ull * i;
-    const uint8_t* pub = pubs + (kKind == 1 ? 32ull : 33ull) * i;
-    const uint8_t* sig = sigs + 64ull * i;
-    if (ok) {
-        Sc s;
-        ok = fp_parse_sig<kKind>(r, s, sig) && fp_parse_key<kKind>(px, odd, pub);
-        if (ok) fp_scalars<kKind>(a, b, r, s, msg, pub, sig);
-    }
-    Fd c, den, zc;
-    JacD A;
-    bool plain = false;      // left to the plain verification
-    __syncthreads();
-    if (ok) {
-        GlvSplit split;
-        glv_split(split, b);
-        eis_recode(dig, split);
-        Fd kx, ky;
-        iso_key(kx, ky, c, px);
-        zc = eis_table(tab, kx, ky);
-    }
-    jacd_set_inf(A);
-    __syncthreads();
-    UF_NOUNROLL
-    for (int q = kEisDigits - 1; q >= 0; --q) {
-        if (ok) eis_add_digit<false>(A, dig[q], q == kEisDigits - 1, tab);
-    }
-    __syncthreads();
-    if (ok) {
-        A.Z = fdc_mul(A.Z, zc);
-        if (kKind == 1) {
-            // the scalar and r again from the signature: not held over the main loop
-            uint32_t sw[8];
-            load_words8(sw, sig + 32);
-            words_be_to_limbs(a.v, sw);
-        }
-        const JacD B = comb_mul<false>(a, comb);
-        if (kKind == 1) {
-            uint32_t sw[8];
-            load_words8(sw, sig);
-            words_be_to_limbs(r, sw);
-        }
-        plain = !iso_prepare<kKind == 1>(tab, den, A, B, c, r);
-    }
-    __syncthreads();
-    if (ok && !plain) {
-        Fe inv;
-        fd_pack(inv.v, den);
-        if (is_zero256(inv.v)) {
-            plain = true;
-        } else {
-            fe_inv(inv, inv);
-            ok = iso_finish<kKind == 1>(tab, inv, odd);
-            // x(R) may be r + n: the plain check looks at both
-            if (kKind != 1 && !ok && r_below_p_minus_n(r)) ok = plain = true;
-        }
-    }
-    if (ok && plain) ok = plain_verify<kKind>(msg, pub, sig, gt, smem + threadIdx.x, blockDim.x);
+    const bool ok = fp_verify<kKind, false>(msgs + 32ull * i, pubs + (kKind == 1 ? 32ull : 33ull) * i, sigs + 64ull * i,
+                                            i < n, nullptr, gt, comb, smem);
     if (i < n) {
         if (collect) {
             if (ok) out[i] = 0;

@@ -2,13 +2,13 @@
 //
 // No reference counterpart (the reference CPU keeps a 1024-slot lift_x cache,
 // src/cpu/src/schnorr.cpp:275, and rebuilds every GPU table per signature).
-// Per distinct key (x, y parity) a slot holds the 1P..8P affine table the
-// verify kernels would otherwise build per signature, so a repeated key skips
-// its square root, its table additions and the table's inversion.
+// Per distinct key (x, y parity) a slot holds the affine 11-point table (eis.cuh)
+// the verify kernels would otherwise build per signature.
 //
-// The table is filled in separate passes ahead of the verify kernels, so that
-// the verify warps never mix lanes that build a table with lanes that copy one
-// (the per-lane lookup inside the verify made 73 % of warps pay both):
+// The table is filled in separate passes ahead of the verify kernels (beside
+// them in small launches, which do not read it), so that the verify warps seldom
+// mix lanes that build a table with lanes that copy one (the per-lane lookup
+// inside the verify made 73 % of warps pay both):
 //
 //   resolve (one thread per item): parse the key, hash it, probe up to
 //     kKeyProbes slots.  An empty slot is claimed (EMPTY -> CLAIMED by
@@ -33,22 +33,6 @@
 
 namespace uf {
 
-#if defined(__CUDACC__)
-#define UF_MEMBER __host__ __device__ __forceinline__
-#else
-#define UF_MEMBER inline
-#endif
-
-// fetch() results: the key's table was loaded / no table (verify the plain
-// way) / the key is known not to be on the curve.
-enum : int { kKeyTable = 1, kKeyNone = 0, kKeyBad = -1 };
-
-// No cache: every key is decompressed and its table built.
-struct NoPubCache {
-    template <class Tab>
-    UF_MEMBER int fetch(Tab&) const { return kKeyNone; }
-};
-
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 
 }  // namespace uf
@@ -62,9 +46,9 @@ struct alignas(64) PubCacheSlot {
     uint32_t state;      // kSlotEmpty .. kSlotBad
     uint32_t key[9];     // x limbs, parity
     uint32_t pad[6];
-    uint4 tab[32];       // entry k: x (2 x uint4), y (2 x uint4)
+    uint4 tab[44];       // entry k of the path in eis.cuh: x (2 x uint4), y (2 x uint4); entry 0 is the key
 };
-static_assert(sizeof(PubCacheSlot) == 576, "slot layout");
+static_assert(sizeof(PubCacheSlot) == 768, "slot layout");
 
 enum : uint32_t { kSlotEmpty = 0, kSlotClaimed = 1, kSlotKeyed = 2, kSlotReady = 3, kSlotBad = 4 };
 constexpr int kKeyProbes = 8;
@@ -136,49 +120,6 @@ __device__ __forceinline__ uint32_t key_lookup(const PubCacheSlot* slots, uint32
     }
     return kNoSlot;
 }
-
-// The verify kernels' view of an item's slot (resolved before the launch).
-struct SlotPubCache {
-    const PubCacheSlot* slot;   // null: no slot
-    template <class Tab>
-    __device__ __noinline__ int fetch(Tab& tab) const {
-        if (!slot) return kKeyNone;
-        const uint32_t st = slot_state(*slot);
-        if (st == kSlotBad) return kKeyBad;
-        if (st != kSlotReady) return kKeyNone;
-        for (int k = 0; k < 8; ++k) {
-            const uint4 a = slot->tab[4 * k], b = slot->tab[4 * k + 1], c = slot->tab[4 * k + 2],
-                        d = slot->tab[4 * k + 3];
-            Fe tx, ty;
-            tx.v[0] = a.x; tx.v[1] = a.y; tx.v[2] = a.z; tx.v[3] = a.w;
-            tx.v[4] = b.x; tx.v[5] = b.y; tx.v[6] = b.z; tx.v[7] = b.w;
-            ty.v[0] = c.x; ty.v[1] = c.y; ty.v[2] = c.z; ty.v[3] = c.w;
-            ty.v[4] = d.x; ty.v[5] = d.y; ty.v[6] = d.z; ty.v[7] = d.w;
-            tab.store(k, tx, ty);
-        }
-        return kKeyTable;
-    }
-};
-
-// A slot's table as the Tab of build_ptable (the build pass writes it in place).
-struct SlotTab {
-    PubCacheSlot* slot;
-    __device__ __forceinline__ void store(int k, const Fe& x, const Fe& y) const {
-        uint4* q = slot->tab + 4 * k;
-        q[0] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-        q[1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
-        q[2] = make_uint4(y.v[0], y.v[1], y.v[2], y.v[3]);
-        q[3] = make_uint4(y.v[4], y.v[5], y.v[6], y.v[7]);
-    }
-    __device__ __forceinline__ void load(int k, Fe& x, Fe& y) const {
-        const uint4* q = slot->tab + 4 * k;
-        const uint4 a = q[0], b = q[1], c = q[2], d = q[3];
-        x.v[0] = a.x; x.v[1] = a.y; x.v[2] = a.z; x.v[3] = a.w;
-        x.v[4] = b.x; x.v[5] = b.y; x.v[6] = b.z; x.v[7] = b.w;
-        y.v[0] = c.x; y.v[1] = c.y; y.v[2] = c.z; y.v[3] = c.w;
-        y.v[4] = d.x; y.v[5] = d.y; y.v[6] = d.z; y.v[7] = d.w;
-    }
-};
 
 }  // namespace uf
 #endif  // __CUDACC__

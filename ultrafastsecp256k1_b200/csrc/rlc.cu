@@ -20,6 +20,7 @@
 #include "keytable.h"
 #include "sign.cuh"
 #include "grpinv.cuh"
+#include "pubcache.cuh"
 #include "verify.cuh"
 #include "nvtx.h"
 #include "rlc_dev.cuh"

@@ -42,7 +42,7 @@ struct ServerConfig {
     uint32_t max_launch_items = 1u << 16;
     uint64_t memory_budget_bytes = 8ull << 30;
     uint32_t batch_window_us = 0;     // wait this long for more work before launching a small batch
-    uint32_t key_cache_log2 = 18;     // resident key table of 2^k slots (576 B each); 0 = none
+    uint32_t key_cache_log2 = 18;     // resident key table of 2^k slots (768 B each); 0 = none
 };
 
 struct ServerStats {

@@ -62,22 +62,16 @@ UF_HDI bool schnorr_check(const Jac& R, const uint32_t r[8]) {
     return diff == 0;
 }
 
-// ECDSA after the signature's scalars are parsed (r, s in [1, n-1]).  `cache`
-// (SlotPubCache / NoPubCache, pubcache.cuh) may supply the key's table instead
-// of decompressing the key and building it, or know the key to be off the
-// curve.
-template <class Tab, class GT, class Cache = NoPubCache>
+// ECDSA after the signature's scalars are parsed (r, s in [1, n-1]).
+template <class Tab, class GT>
 UF_HDI bool ecdsa_verify_rs(const uint32_t msg_w[8], const uint8_t* pub33, const Sc& r, const Sc& s, Tab& tab,
-                            const GT& gt, const Cache& cache = Cache()) {
+                            const GT& gt) {
     const uint8_t prefix = pub33[0];
     if (prefix != 0x02 && prefix != 0x03) return false;
     Fe qx, qy;
     be32_to_limbs(qx.v, pub33 + 1);
     if (!limbs_lt_p(qx.v)) return false;
-    const int c = cache.fetch(tab);
-    if (c == kKeyBad) return false;
-    const bool cached = c == kKeyTable;
-    if (!cached && !lift_x_parity(qy, qx, prefix == 0x03)) return false;
+    if (!lift_x_parity(qy, qx, prefix == 0x03)) return false;
     Sc z, w, u1, u2;
     words_be_to_limbs(z.v, msg_w);
     sc_reduce_once(z);
@@ -85,22 +79,22 @@ UF_HDI bool ecdsa_verify_rs(const uint32_t msg_w[8], const uint8_t* pub33, const
     sc_mul(u1, z, w);
     sc_mul(u2, r, w);
     Jac R;
-    dual_mul_c(R, u1, qx, qy, u2, tab, gt, cached);
+    dual_mul(R, u1, qx, qy, u2, tab, gt);
     return ecdsa_check_x(R, r);
 }
 
 // msg_w / sig_w: the 32 / 64 input bytes as words loaded little-endian;
 // compact big-endian r || s, low-S required.
-template <class Tab, class GT, class Cache = NoPubCache>
+template <class Tab, class GT>
 UF_HDI bool ecdsa_verify_one(const uint32_t msg_w[8], const uint8_t* pub33, const uint32_t sig_w[16],
-                             Tab& tab, const GT& gt, const Cache& cache = Cache()) {
+                             Tab& tab, const GT& gt) {
     Sc r, s;
     words_be_to_limbs(r.v, sig_w);
     words_be_to_limbs(s.v, sig_w + 8);
     if (sc_is_zero(r) || !limbs_lt_n(r.v)) return false;
     if (sc_is_zero(s) || !limbs_lt_n(s.v)) return false;
     if (!sc_is_low(s.v)) return false;
-    return ecdsa_verify_rs(msg_w, pub33, r, s, tab, gt, cache);
+    return ecdsa_verify_rs(msg_w, pub33, r, s, tab, gt);
 }
 
 // The libsecp in-memory signature layout of the consensus surfaces
@@ -123,9 +117,9 @@ UF_HDI bool ecdsa_verify_opaque_one(const uint32_t msg_w[8], const uint8_t* pub3
     return ecdsa_verify_rs(msg_w, pub33, r, s, tab, gt);
 }
 
-template <class Tab, class GT, class Cache = NoPubCache>
+template <class Tab, class GT>
 UF_HDI bool schnorr_verify_one(const uint32_t msg_w[8], const uint32_t px_w[8], const uint32_t sig_w[16],
-                               Tab& tab, const GT& gt, const Cache& cache = Cache()) {
+                               Tab& tab, const GT& gt) {
     uint32_t r[8];
     Sc s;
     words_be_to_limbs(r, sig_w);
@@ -135,10 +129,7 @@ UF_HDI bool schnorr_verify_one(const uint32_t msg_w[8], const uint32_t px_w[8], 
     Fe px, py;
     words_be_to_limbs(px.v, px_w);
     if (!limbs_lt_p(px.v)) return false;
-    const int c = cache.fetch(tab);
-    if (c == kKeyBad) return false;
-    const bool cached = c == kKeyTable;
-    if (!cached && !lift_x_parity(py, px, false)) return false;
+    if (!lift_x_parity(py, px, false)) return false;
     uint32_t rbe[8], pbe[8], mbe[8], h[8];
     UF_UNROLL
     for (int i = 0; i < 8; ++i) {
@@ -153,7 +144,7 @@ UF_HDI bool schnorr_verify_one(const uint32_t msg_w[8], const uint32_t px_w[8], 
     sc_reduce_once(e);
     sc_neg(ne, e);
     Jac R;
-    dual_mul_c(R, s, px, py, ne, tab, gt, cached);
+    dual_mul(R, s, px, py, ne, tab, gt);
     return schnorr_check(R, r);
 }
 

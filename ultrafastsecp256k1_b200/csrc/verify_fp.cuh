@@ -1,8 +1,9 @@
-// Pieces shared by the verify kernels on the FP64 pipe (kernels_verify_fp.cu,
-// kernels_team.cu).
+// The verify kernels' body on the FP64 pipe (kernels_verify_fp.cu, kernels_queue.cu)
+// and the pieces it shares with the small-call form (team.cuh).
 #pragma once
 #include "dev_tables.cuh"
 #include "isocheck.cuh"
+#include "pubcache.cuh"
 #include "verify.cuh"
 
 #if defined(__CUDACC__)
@@ -126,6 +127,98 @@ __device__ __forceinline__ void fp_scalars(Sc& a, Sc& b, const uint32_t r[8], co
         sc_mul(a, z, w);
         sc_mul(b, rs, w);
     }
+}
+
+// One item per thread; every thread of the block calls it (ok false for threads
+// without one, whose pointers are not read).  smem: blockDim.x point tables.
+// The barriers keep the block's warps at the same place in the code and serve
+// nothing else.  kCached: `slot` may hold the key's table (pubcache.cuh); null
+// or a slot that is not ready yet: the key's table is built here.
+template <int kKind, bool kCached>
+__device__ __forceinline__ bool fp_verify(const uint8_t* msg, const uint8_t* pub, const uint8_t* sig, bool ok,
+                                          const PubCacheSlot* slot, const uint4* gt, const uint4* comb, uint4* smem) {
+    const EisTab tab{reinterpret_cast<double2*>(smem) + threadIdx.x, blockDim.x};
+    bool odd = false;
+    uint32_t px[8], r[8];
+    Sc a, b;             // R = a G + b P
+    uint8_t dig[kEisDigits];
+    if (ok) {
+        Sc s;
+        ok = fp_parse_sig<kKind>(r, s, sig) && fp_parse_key<kKind>(px, odd, pub);
+        if (ok) fp_scalars<kKind>(a, b, r, s, msg, pub, sig);
+    }
+    Fd c, den, zc;
+    JacD A;
+    bool plain = false;      // left to the plain verification
+    bool unit = false;       // the key's table comes from its slot
+    if (kCached && ok && slot) {
+        const uint32_t st = slot_state(*slot);
+        unit = st == kSlotReady;
+        if (st == kSlotBad) ok = false;
+    }
+    __syncthreads();
+    if (ok) {
+        GlvSplit split;
+        glv_split(split, b);
+        eis_recode(dig, split);
+        if (kCached && unit) {
+            UF_NOUNROLL
+            for (int k = 0; k < kEisTab; ++k) {
+                const uint4 x0 = slot->tab[4 * k], x1 = slot->tab[4 * k + 1], y0 = slot->tab[4 * k + 2],
+                            y1 = slot->tab[4 * k + 3];
+                const uint32_t xw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+                const uint32_t yw[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+                Fd x, y;
+                fd_unpack(x, xw);
+                fd_unpack(y, yw);
+                tab.store(k, x, y);
+            }
+            fd_set_u32(c, 1);
+            fd_set_u32(zc, 1);
+        } else {
+            Fd kx, ky;
+            iso_key(kx, ky, c, px);
+            zc = eis_table(tab, kx, ky);
+        }
+    }
+    jacd_set_inf(A);
+    __syncthreads();
+    UF_NOUNROLL
+    for (int q = kEisDigits - 1; q >= 0; --q) {
+        if (ok) eis_add_digit<false>(A, dig[q], q == kEisDigits - 1, tab);
+    }
+    __syncthreads();
+    if (ok) {
+        A.Z = fdc_mul(A.Z, zc);
+        if (kKind == 1) {
+            // the scalar and r again from the signature: not held over the main loop
+            uint32_t sw[8];
+            load_words8(sw, sig + 32);
+            words_be_to_limbs(a.v, sw);
+        }
+        const JacD B = comb_mul<false>(a, comb);
+        if (kKind == 1) {
+            uint32_t sw[8];
+            load_words8(sw, sig);
+            words_be_to_limbs(r, sw);
+        }
+        plain = !iso_prepare<kKind == 1>(tab, den, A, B, c, r);
+    }
+    __syncthreads();
+    if (ok && !plain) {
+        Fe inv;
+        fd_pack(inv.v, den);
+        if (is_zero256(inv.v)) {
+            plain = true;
+        } else {
+            fe_inv(inv, inv);
+            ok = iso_finish<kKind == 1>(tab, inv, odd, unit);
+            // x(R) may be r + n: the plain check looks at both
+            if (kKind != 1 && !ok && r_below_p_minus_n(r)) ok = plain = true;
+        }
+    }
+    if (ok && plain) ok = plain_verify<kKind>(msg, pub, sig, gt, smem + threadIdx.x, blockDim.x);
+    return ok;
 }
 
 }  // namespace uf
