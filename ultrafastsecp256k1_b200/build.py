@@ -65,9 +65,7 @@ VARIANTS = {"kernels_verify.cu": _VARIANT_FLAGS + _WINDOW_FLAGS, "kernels_probe.
             "kernels_queue.cu": [("", _BEST_FLAGS)], "kernels_noalloc.cu": [("", _BEST_FLAGS)],
             "kernels_verify_fp.cu": [("", _BEST_FLAGS)], "kernels_team.cu": [("", _BEST_FLAGS)],
             "rlc.cu": [("", _BEST_FLAGS)], "kernels_ops.cu": [("", _BEST_FLAGS)],
-            # the RLC kernels with one serial chain per segment or window run few
-            # threads: field and point operations inlined, for overlap inside a chain
-            "rlc_serial.cu": [("", ["-DUF_PTX_MUL"])]}
+            "rlc_serial.cu": [("", _BEST_FLAGS)]}
 
 
 def _sources():

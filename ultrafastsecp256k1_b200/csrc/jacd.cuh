@@ -91,6 +91,77 @@ UF_HD JacD jacd_add_aff_t(JacD a, Fd x2, Fd y2) {
 
 UF_COLD JacD jacd_add_aff(JacD a, Fd x2, Fd y2) { return jacd_add_aff_t<false>(a, x2, y2); }
 
+// (X, Y, ZZ = Z^2, ZZZ = Z^3): for long runs of mixed additions, one squaring
+// less each than in Jacobian form.
+struct XyzzD { Fd X, Y, ZZ, ZZZ; bool inf; };
+
+UF_HD void xyzzd_set_inf(XyzzD& a) {
+    fd_set_u32(a.X, 0);
+    fd_set_u32(a.Y, 1);
+    fd_set_u32(a.ZZ, 0);
+    fd_set_u32(a.ZZZ, 0);
+    a.inf = true;
+}
+
+// 2 (x, y) of an affine point, strict digits.
+UF_COLD XyzzD xyzzd_dbl_aff(Fd x, Fd y) {
+    XyzzD r;
+    const Fd M = fd_sqr_x<3>(x), H = fd_sqr_x<2>(y);       // 3 x^2, 2 y^2
+    r.ZZ = fd_add_l(H, H);                                 // (2 y)^2
+    fd_strict(r.ZZ);
+    r.ZZZ = fdc_mul(fd_add_l(y, y), r.ZZ);
+    const Fd S = fdc_mul(x, r.ZZ);
+    r.X = fd_sqr_sub2(M, S);
+    r.Y = fdc_mul_sub(fd_sub_l(S, r.X), M, fdc_mul(y, r.ZZZ));
+    r.inf = false;
+    return r;
+}
+
+// a += (x2, y2), digits as in jacd_add_aff_t, exact for every input: 8M + 2S, the
+// products of Y3 reduced together.
+UF_HD void xyzzd_add_aff(XyzzD& a, Fd x2, Fd y2) {
+    if (a.inf) {
+        fd_strict(x2);
+        fd_strict(y2);
+        a.X = x2;
+        a.Y = y2;
+        fd_set_u32(a.ZZ, 1);
+        fd_set_u32(a.ZZZ, 1);
+        a.inf = false;
+        return;
+    }
+    const Fd H = fd_mul_sub(x2, a.ZZ, a.X);
+    const Fd r = fd_mul_sub(y2, a.ZZZ, a.Y);
+    if (fd_is_zero(H)) {
+        if (fd_is_zero(r)) {
+            fd_strict(x2);
+            fd_strict(y2);
+            a = xyzzd_dbl_aff(x2, y2);
+        } else {
+            a.inf = true;
+        }
+        return;
+    }
+    const Fd HH = fd_sqr(H);
+    const Fd HHH = fd_mul(H, HH);
+    const Fd V = fd_mul(a.X, HH);
+    a.ZZ = fd_mul(a.ZZ, HH);
+    a.ZZZ = fd_mul(a.ZZZ, HHH);
+    a.X = fd_sqr_sub_sub2(r, HHH, V);
+    a.Y = fd_mul_mul_sub(fd_sub_l(V, a.X), r, a.Y, HHH);
+}
+
+// The same point in Jacobian form: Z' = Z ZZ = ZZZ, so X' = X ZZ^2, Y' = Y ZZ^3.
+UF_HD JacD xyzzd_to_jac(const XyzzD& a) {
+    JacD p;
+    const Fd w = fdc_sqr(a.ZZ);
+    p.X = fdc_mul(a.X, w);
+    p.Y = fdc_mul(a.Y, fdc_mul(w, a.ZZ));
+    p.Z = a.ZZZ;
+    p.inf = a.inf;
+    return p;
+}
+
 // General addition, exact for every input (a few per signature).
 UF_COLD JacD jacd_add(JacD a, JacD b) {
     if (b.inf) return a;

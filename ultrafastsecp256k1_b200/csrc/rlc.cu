@@ -41,9 +41,11 @@ struct RlcSeed {
 };
 
 // Running sums of a window's B buckets are split into S sub-ranges of B / S
-// buckets (one thread each) and the S partial results are combined by one
-// thread; S = 2^floor((c - 1) / 2) balances the two serial chains.
-inline int sub_ranges(int c) { return 1 << ((c - 1) / 2); }
+// buckets (one thread each) and the S partial results joined by a tree over S
+// lanes, at most a warp.  Narrow windows (c <= 8) come with many segments, which
+// fill the device: S = 2^floor((c - 1) / 2); for wider ones the chain of B / S
+// additions is what counts: S = 32.
+inline int sub_ranges(int c) { return c >= 9 ? 32 : 1 << ((c - 1) / 2); }
 
 // Signed digit of window w (c bits) of a magnitude m + hi 2^128 < 2^160 (the
 // recoding of booth_recode in ecmult.cuh with a run-time window width).
@@ -63,6 +65,12 @@ __device__ __forceinline__ int booth_digit(const uint4 m, uint32_t hi, int w, in
 }
 
 // Point pidx of the round: 3 per item, then G / lambda G per segment.
+__device__ __forceinline__ const uint4* point_of(uint32_t pidx, const RlcItem* __restrict__ items, uint32_t n3,
+                                                 const uint4* __restrict__ gt) {
+    if (pidx < n3) return items[pidx / 3u].pt[pidx % 3u];
+    return gt + 4 * (size_t)(((pidx - n3) & 1u) ? kGTab : 0);
+}
+
 __device__ __forceinline__ void load_point(uint32_t pidx, const RlcItem* __restrict__ items, uint32_t n3,
                                            const uint4* __restrict__ gt, Fe& x, Fe& y) {
     if (pidx < n3) {
@@ -300,7 +308,7 @@ __global__ void k_rlc_nchunks(const uint32_t* __restrict__ counts, uint32_t K, u
 
 // One thread per chunk of at most `chunk` entries of one bucket.  A bucket
 // with a single chunk is written straight to its bucket slot.
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 2)
 k_rlc_chunks(const uint32_t* __restrict__ coff, uint32_t K, uint32_t chunk, const uint32_t* __restrict__ offsets,
              const uint32_t* __restrict__ entries, const RlcItem* __restrict__ items, uint32_t n3,
              const uint4* __restrict__ gt, uint4* __restrict__ partials, uint4* __restrict__ buckets) {
@@ -310,17 +318,31 @@ k_rlc_chunks(const uint32_t* __restrict__ coff, uint32_t K, uint32_t chunk, cons
     const uint32_t j = t - coff[key];
     const uint32_t e0 = offsets[key] + j * chunk;
     const uint32_t e1 = min(e0 + chunk, offsets[key + 1]);
-    Jac acc;
-    jac_set_inf(acc);
+    XyzzD acc;
+    xyzzd_set_inf(acc);
+    // the next entry's point is fetched while this one is added
+    uint32_t v = entries[e0];
+    const uint4* q = point_of(v & 0x7FFFFFFFu, items, n3, gt);
+    uint4 p0 = q[0], p1 = q[1], p2 = q[2], p3 = q[3];
     for (uint32_t e = e0; e < e1; ++e) {
-        const uint32_t v = entries[e];
-        Fe x, y;
-        load_point(v & 0x7FFFFFFFu, items, n3, gt, x, y);
-        if (v >> 31) fe_neg(y, y);
-        jac_add_aff(acc, x, y);
+        const uint32_t xw[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+        const uint32_t yw[8] = {p2.x, p2.y, p2.z, p2.w, p3.x, p3.y, p3.z, p3.w};
+        Fd x, y;
+        fd_unpack(x, xw);
+        fd_unpack(y, yw);
+        const double sg = v >> 31 ? -1.0 : 1.0;
+        UF_UNROLL
+        for (int k = 0; k < 5; ++k) y.v[k] *= sg;
+        if (e + 1 < e1) {
+            v = entries[e + 1];
+            q = point_of(v & 0x7FFFFFFFu, items, n3, gt);
+            p0 = q[0]; p1 = q[1]; p2 = q[2]; p3 = q[3];
+        }
+        xyzzd_add_aff(acc, x, y);
     }
-    if (coff[key + 1] - coff[key] == 1) store_jac(buckets + kJacQ * (uint64_t)key, acc);
-    else store_jac(partials + kJacQ * (uint64_t)t, acc);
+    const JacD sum = xyzzd_to_jac(acc);
+    if (coff[key + 1] - coff[key] == 1) store_jacd(buckets + kJacQ * (uint64_t)key, sum);
+    else store_jacd(partials + kJacQ * (uint64_t)t, sum);
 }
 
 // ------------------------------------------------- batch-affine chunk sums --

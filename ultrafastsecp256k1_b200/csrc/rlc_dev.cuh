@@ -3,6 +3,7 @@
 #pragma once
 #include "common.cuh"
 #include "fe.cuh"
+#include "jacd.cuh"
 #include "point.cuh"
 
 namespace uf {
@@ -39,6 +40,36 @@ __device__ __forceinline__ void load_jac(const uint4* q, Jac& P) {
     P.Z.v[0] = a.x; P.Z.v[1] = a.y; P.Z.v[2] = a.z; P.Z.v[3] = a.w;
     P.Z.v[4] = b.x; P.Z.v[5] = b.y; P.Z.v[6] = b.z; P.Z.v[7] = b.w;
     P.inf = q[6].x != 0;
+}
+
+// The same storage for points in digit form (jacd.cuh): any 256-bit representative
+// is read, canonical ones are written where the point was computed in that form.
+__device__ __forceinline__ void load_limbs(Fd& r, const uint4* q) {
+    const uint4 a = q[0], b = q[1];
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    fd_unpack(r, w);
+    fd_strict(r);
+}
+
+__device__ __forceinline__ void store_limbs(uint4* q, const Fd& a) {
+    uint32_t w[8];
+    fd_pack(w, a);
+    q[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    q[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+__device__ __forceinline__ void load_jacd(const uint4* q, JacD& p) {
+    load_limbs(p.X, q);
+    load_limbs(p.Y, q + 2);
+    load_limbs(p.Z, q + 4);
+    p.inf = q[6].x != 0;
+}
+
+__device__ __forceinline__ void store_jacd(uint4* q, const JacD& p) {
+    store_limbs(q, p.X);
+    store_limbs(q + 2, p.Y);
+    store_limbs(q + 4, p.Z);
+    q[6] = make_uint4(p.inf ? 1u : 0u, 0u, 0u, 0u);
 }
 
 // Round geometry in device memory: seg[2s], seg[2s+1] = first item, length of
