@@ -115,12 +115,6 @@ public:
     // the tuning file's rlc_locate or UFSECP_B200_RLC_LOCATE may turn it off.
     bool rlc_locate() const { return rlc_locate_; }
     void set_rlc_locate(bool on) { rlc_locate_ = on; }
-    // Whether RLC bucket chunks (of at most 16 points) are summed by affine
-    // pairwise trees with grid-shared inversions (k_aff_fwd / k_aff_bwd)
-    // instead of mixed Jacobian additions (k_rlc_chunks).  On by default; the
-    // tuning file's rlc_affine or UFSECP_B200_RLC_AFFINE may turn it off.
-    bool rlc_affine() const { return rlc_affine_; }
-    void set_rlc_affine(bool on) { rlc_affine_ = on; }
     // Mixed-job launches of at most this many items (both kinds together) run
     // four warps per 32 signatures: the smaller of the kinds' limits.
     uint32_t queue_pair_items() const { return std::min(pair_items_[0], pair_items_[1]); }
@@ -235,7 +229,6 @@ private:
     std::map<uint32_t, uint32_t> rlc_chunk_;  // tuned bucket points per chunk thread per RLC batch size
     uint32_t rlc_chunk_fixed_ = 0;            // set_rlc_chunk / UFSECP_B200_RLC_CHUNK override, 0 = tuned
     bool rlc_locate_ = true;
-    bool rlc_affine_ = true;
     int last_err_ = kOk;
     std::string last_msg_ = "OK";
     std::atomic<long long> fault_after_{-1};

@@ -109,22 +109,12 @@ k_rlc_finish(RoundGeo g, const uint4* __restrict__ wins, const uint32_t* __restr
 // A bucket of more than kHeavyChunks chunks (skewed digits: the top windows
 // of a locate round's j-scaled magnitudes put most points of a segment into a
 // few buckets) is left to k_rlc_bucket_heavy: its key goes to `heavy`.
-// Adds a chunk partial: affine (Z = 1, from the affine chunk trees) or Jacobian.
-template <bool kAff>
 __device__ __forceinline__ void add_partial(JacD& acc, const uint4* q) {
-    if (!kAff) {
-        JacD p;
-        load_jacd(q, p);
-        acc = jacd_add(acc, p);
-    } else if (q[6].x == 0) {
-        Fd x, y;
-        load_limbs(x, q);
-        load_limbs(y, q + 2);
-        acc = jacd_add_aff(acc, x, y);
-    }
+    JacD p;
+    load_jacd(q, p);
+    acc = jacd_add(acc, p);
 }
 
-template <bool kAff>
 __global__ void __launch_bounds__(128)
 k_rlc_bucket_fin(const uint32_t* __restrict__ coff, uint32_t K, const uint4* __restrict__ partials,
                  uint4* __restrict__ buckets, uint32_t* __restrict__ heavy) {
@@ -138,14 +128,13 @@ k_rlc_bucket_fin(const uint32_t* __restrict__ coff, uint32_t K, const uint4* __r
     }
     JacD acc;
     jacd_set_inf(acc);
-    for (uint32_t c = c0; c < c1; ++c) add_partial<kAff>(acc, partials + kJacQ * (uint64_t)c);
+    for (uint32_t c = c0; c < c1; ++c) add_partial(acc, partials + kJacQ * (uint64_t)c);
     store_jacd(buckets + kJacQ * (uint64_t)k, acc);
 }
 
 // One warp per heavy bucket (heavy[0] of them, keys in heavy[1..]): lane l
 // sums partials l, l + 32, ..., then the 32 lane sums meet in a shuffle tree:
 // about chunks / 32 + 5 serial additions instead of chunks.
-template <bool kAff>
 __global__ void __launch_bounds__(128)
 k_rlc_bucket_heavy(const uint32_t* __restrict__ coff, const uint4* __restrict__ partials,
                    uint4* __restrict__ buckets, const uint32_t* __restrict__ heavy) {
@@ -156,12 +145,40 @@ k_rlc_bucket_heavy(const uint32_t* __restrict__ coff, const uint4* __restrict__ 
         const uint32_t c0 = coff[k], c1 = coff[k + 1];
         JacD acc;
         jacd_set_inf(acc);
-        for (uint32_t c = c0 + lane; c < c1; c += 32) add_partial<kAff>(acc, partials + kJacQ * (uint64_t)c);
+        for (uint32_t c = c0 + lane; c < c1; c += 32) add_partial(acc, partials + kJacQ * (uint64_t)c);
         for (int o = 16; o > 0; o >>= 1) {
             const JacD other = shfl_jacd(acc, (int)(lane ^ (uint32_t)o));
             acc = jacd_add(acc, other);
         }
         if (lane == 0) store_jacd(buckets + kJacQ * (uint64_t)k, acc);
+    }
+}
+
+constexpr uint64_t kWarpHornerSegments = 592;      // one warp per scheduler of a 148-SM device
+
+// The same with a warp per segment (at most 32 windows): lane w doubles window
+// w's sum c w times, all windows at once, and a tree adds them: the chain has the
+// same doublings but log2(W) additions instead of W - 1.  For rounds of few
+// segments; many fill the device with a thread each.
+__global__ void __launch_bounds__(32)
+k_rlc_finish_warp(RoundGeo g, const uint4* __restrict__ wins, const uint32_t* __restrict__ segbad,
+                  uint8_t* __restrict__ segok, uint4* __restrict__ segpt) {
+    const uint32_t s = blockIdx.x;
+    const int lane = (int)threadIdx.x;
+    JacD acc;
+    jacd_set_inf(acc);
+    if (lane < g.W) {
+        load_jacd(wins + kJacQ * ((uint64_t)s * g.W + lane), acc);
+        acc = jacd_dbl_n(acc, g.c * lane);
+    }
+    __syncwarp();
+    for (int d = 1; d < g.W; d <<= 1) {
+        const JacD o = shfl_jacd(acc, lane + d < 32 ? lane + d : lane);
+        if (lane + d < 32) acc = jacd_add(acc, o);
+    }
+    if (lane == 0) {
+        segok[s] = (uint8_t)((acc.inf ? 1 : 0) | (segbad[s] ? 2 : 0));
+        store_jacd(segpt + kJacQ * (uint64_t)s, acc);
     }
 }
 
@@ -174,19 +191,17 @@ cudaError_t launch_rlc_windows(const RoundGeo& g, const uint4* buckets, uint4* w
     const uint64_t n_seg = g.n_seg;
     k_rlc_wpart<<<grid_of(n_seg * g.W * g.S, 128), 128, 0, s>>>(g, buckets, wu, wt);
     k_rlc_wcomb<<<grid_of(n_seg * g.W * g.S, 128), 128, 0, s>>>(g, wu, wt, wins);
-    k_rlc_finish<<<grid_of(n_seg, 32), 32, 0, s>>>(g, wins, segbad, segok, segpt);
+    if (g.W <= 32 && n_seg <= kWarpHornerSegments)
+        k_rlc_finish_warp<<<(unsigned)n_seg, 32, 0, s>>>(g, wins, segbad, segok, segpt);
+    else
+        k_rlc_finish<<<grid_of(n_seg, 32), 32, 0, s>>>(g, wins, segbad, segok, segpt);
     return cudaGetLastError();
 }
 
-cudaError_t launch_rlc_bucket_merge(bool affine, const uint32_t* coff, uint32_t K, const uint4* partials,
-                                    uint4* buckets, uint32_t* heavy, int heavy_grid, cudaStream_t s) {
-    if (affine) {
-        k_rlc_bucket_fin<true><<<grid_of(K, 128), 128, 0, s>>>(coff, K, partials, buckets, heavy);
-        k_rlc_bucket_heavy<true><<<heavy_grid, 128, 0, s>>>(coff, partials, buckets, heavy);
-    } else {
-        k_rlc_bucket_fin<false><<<grid_of(K, 128), 128, 0, s>>>(coff, K, partials, buckets, heavy);
-        k_rlc_bucket_heavy<false><<<heavy_grid, 128, 0, s>>>(coff, partials, buckets, heavy);
-    }
+cudaError_t launch_rlc_bucket_merge(const uint32_t* coff, uint32_t K, const uint4* partials, uint4* buckets,
+                                    uint32_t* heavy, int heavy_grid, cudaStream_t s) {
+    k_rlc_bucket_fin<<<grid_of(K, 128), 128, 0, s>>>(coff, K, partials, buckets, heavy);
+    k_rlc_bucket_heavy<<<heavy_grid, 128, 0, s>>>(coff, partials, buckets, heavy);
     return cudaGetLastError();
 }
 

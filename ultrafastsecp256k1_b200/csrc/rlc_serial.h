@@ -17,11 +17,10 @@ namespace uf {
 cudaError_t launch_rlc_windows(const rlcdev::RoundGeo& g, const uint4* buckets, uint4* wu, uint4* wt, uint4* wins,
                                const uint32_t* segbad, uint8_t* segok, uint4* segpt, cudaStream_t s);
 
-// Buckets of two or more chunks: the sum of their chunk partials (mixed
-// additions when the partials are affine, else Jacobian), by a thread per
-// bucket, or by a warp per bucket of more than kHeavyChunks chunks (their keys
-// listed in heavy[1..heavy[0]] by the first kernel).
-cudaError_t launch_rlc_bucket_merge(bool affine, const uint32_t* coff, uint32_t K, const uint4* partials,
-                                    uint4* buckets, uint32_t* heavy, int heavy_grid, cudaStream_t s);
+// Buckets of two or more chunks: the sum of their chunk partials, by a thread
+// per bucket, or by a warp per bucket of more than kHeavyChunks chunks (their
+// keys listed in heavy[1..heavy[0]] by the first kernel).
+cudaError_t launch_rlc_bucket_merge(const uint32_t* coff, uint32_t K, const uint4* partials, uint4* buckets,
+                                    uint32_t* heavy, int heavy_grid, cudaStream_t s);
 
 }  // namespace uf
