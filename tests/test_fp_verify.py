@@ -260,3 +260,35 @@ def test_team_block_edges(team_ctx, oracle, n):
 @pytest.mark.gpu
 def test_team_sums_that_meet(team_ctx, oracle):
     check_meeting(team_ctx, oracle)
+
+
+@pytest.fixture(scope="module")
+def plain_ctx():
+    import ultrafastsecp256k1_b200 as uf
+    with uf.GpuContext(0) as ctx:
+        yield ctx
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 37889, 47360, 47361, 56832, 56833, 75809])
+def test_chunks_and_last_waves(plain_ctx, oracle, n):
+    """Host calls around the size from which staging is packed in pieces, and
+    around whole waves (256 items on each of 148 SMs) plus the last waves that
+    run in their own form: up to 64 items per SM, up to 128, and more."""
+    check_sizes(plain_ctx, oracle, n)
+
+
+@pytest.mark.gpu
+def test_jobs_packed_in_pieces(plain_ctx, oracle):
+    em, ep, es = ecdsa_corpus(oracle, 701, 17)
+    sm, sp, ss = schnorr_corpus(oracle, 701, 18, tamper=0.1)
+    rng = np.random.default_rng(5)
+    jobs, want = [], []
+    for k, n in ((1, 9001), (0, 1), (0, 5003), (1, 33), (1, 0), (0, 3000), (1, 4096), (0, 21000), (1, 2)):
+        order = rng.integers(0, 701, n)
+        src = (em, ep, es) if k == 0 else (sm, sp, ss)
+        jobs.append((k, *(np.ascontiguousarray(a[order]) for a in src)))
+        ref = oracle.ecdsa_verify_batch(em, ep, es) if k == 0 else oracle.schnorr_verify_batch(sm, sp, ss)
+        want.append(ref[order])
+    for got, ref in zip(plain_ctx.verify_jobs(jobs), want):
+        assert (got == ref).all()

@@ -16,6 +16,7 @@
 #include "keytable.h"
 #include "kernels.h"
 #include "pack_pool.h"
+#include "stage_copy.h"
 #include "rlc.h"
 #include "nvtx.h"
 
@@ -23,8 +24,7 @@ namespace uf {
 
 namespace {
 // Items per host->device chunk: bounds device memory at ~130 B x 2^22 = 0.5 GB.
-constexpr size_t kPipeChunk = size_t{1} << 17;   // items per staging slot of a host-buffer call
-constexpr size_t kPipeFirst = size_t{1} << 14;   // items in a host-buffer call's first chunk
+constexpr size_t kPackPiece = 1024;              // items a packing thread takes at a time
 constexpr size_t kJobsPipeItems = size_t{1} << 16;   // most items per sub-call of a large mixed-job call
 constexpr size_t kPackSplitItems = size_t{1} << 13;  // chunks at least this large are packed by the pool
 constexpr size_t kDeviceChunk = size_t{1} << 17; // items per launch of a large device-buffer call
@@ -47,13 +47,14 @@ int env_int(const char* name, int dflt) {
 }  // namespace
 
 cudaError_t Backend::launch_verify(int kind, const uint8_t* m, const uint8_t* p, const uint8_t* s, uint32_t n,
-                                   uint8_t* out, int collect, cudaStream_t st, size_t call_items) {
+                                   uint8_t* out, int collect, cudaStream_t st) {
     const int k = kind & 1;
-    if (call_items <= pair_items_[k])
+    if (n <= pair_items_[k])
         return launch_verify_team(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, st);
-    const bool small = small_variant_[k] >= 0 && call_items <= small_items_[k];
-    if (!small && inv_group_[k] > 1)
+    const bool small = small_variant_[k] >= 0 && n <= small_items_[k];
+    if (!small && inv_group_[k] > 1) {
         return launch_verify_fp(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, sms_, st);
+    }
     const int v = small ? small_variant_[k] : variant_[k];
     return kLaunchers[v](kind, m, p, s, n, gtab_for(v), out, collect, grid_[v][k], st);
 }
@@ -394,7 +395,7 @@ int Backend::verify_device(int kind, const uint8_t* d_msgs, const uint8_t* d_pub
     if (count < 2 * kDeviceChunk || inv_group_[kind & 1] > 1) {
         if (count >= 2 * kDeviceChunk)
             if (const int rc = fault_point("verify launch")) return rc;
-        e = launch_verify(kind, d_msgs, d_pubs, d_sigs, (uint32_t)count, d_out, 0, s, count);
+        e = launch_verify(kind, d_msgs, d_pubs, d_sigs, (uint32_t)count, d_out, 0, s);
         if (e != cudaSuccess) return cuda_error(e, "verify launch");
         clear_error();
         return kOk;
@@ -417,7 +418,7 @@ int Backend::verify_device(int kind, const uint8_t* d_msgs, const uint8_t* d_pub
     for (size_t off = 0; off < count; off += kDeviceChunk, ++k) {
         const size_t m = std::min(kDeviceChunk, count - off);
         e = launch_verify(kind, d_msgs + 32 * off, d_pubs + pub_sz * off, d_sigs + 64 * off, (uint32_t)m, d_out + off,
-                          0, (k & 1) ? dstream_ : s, count);
+                          0, (k & 1) ? dstream_ : s);
         if (e != cudaSuccess) return cuda_error(e, "verify launch");
     }
     if ((e = cudaEventRecord(djoin_, dstream_)) != cudaSuccess || (e = cudaStreamWaitEvent(s, djoin_, 0)) != cudaSuccess)
@@ -446,16 +447,19 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         }
         if (e != cudaSuccess) return cuda_error(e, "pipeline streams");
     }
-    // Chunks of up to kPipeChunk items rotate through kPipeSlots pinned
-    // staging slots: the CPU packs chunk k + 2 (and unpacks chunk k - 1's
-    // verdicts) while the device copies in and verifies chunks k and k + 1.  Per chunk the slot is
-    // laid out msgs | keys | sigs (16-byte aligned) | verdicts, copied in and
-    // out with one transfer each way.
+    // A chunk is one wave of the verify kernel (256 items per SM, 37,888 on a
+    // 148-SM B200): a smaller one would take the device as long as a full one
+    // once it holds more than 128 items per SM (0.68 ms; 0.54 below), and the
+    // CPU packs and copies in a wave in 0.2 ms.  Chunks rotate through
+    // kPipeSlots pinned staging slots: the CPU packs chunk k + 2 (and unpacks
+    // chunk k - 1's verdicts) while the device copies in and verifies chunks k
+    // and k + 1.  Per chunk the slot is laid out msgs | keys | sigs (16-byte
+    // aligned) | verdicts.
     const size_t pub_sz = kind == 1 ? 32 : 33;
-    const size_t sub = std::min(count, kPipeChunk);
+    const size_t sub = std::min(count, (size_t)sms_ * 256);
     auto a16 = [](size_t v) { return (v + 15) & ~size_t{15}; };
     const size_t slot_bytes = a16(sub * (32 + pub_sz)) + sub * 64 + sub + 16;
-    const int slots = count > kPipeFirst ? kPipeSlots : 1;   // chunks of the ramp below use every slot
+    const int slots = (int)std::min<size_t>(kPipeSlots, (count + sub - 1) / sub);
     for (int j = 0; j < slots; ++j) {
         if ((e = pstage_[j].ensure(slot_bytes)) != cudaSuccess) return cuda_error(e, "cudaHostAlloc(staging)");
         if ((e = dstage_[j].ensure(slot_bytes)) != cudaSuccess) return cuda_error(e, "cudaMalloc(staging)");
@@ -468,10 +472,6 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         pend_n[j] = 0;
         return r;
     };
-    // Chunk sizes ramp up from kPipeFirst, doubling to kPipeChunk: the
-    // pipeline's fill (packing and copying the first chunk while the device
-    // is idle) costs a small chunk, and the device fills up while the CPU
-    // packs the next, larger ones.
     // every early return waits for the slots' streams first, so that no copy
     // of this call is still in flight when the next call packs a slot
     auto fail = [&](int rc) {
@@ -485,36 +485,43 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         const int j = (int)(k % kPipeSlots);
         if ((e = drain(j)) != cudaSuccess) return fail(cuda_error(e, "verify"));
         if (const int rc = fault_point("verify launch")) return fail(rc);
-        m = std::min(std::min(sub, kPipeFirst << std::min<size_t>(k, 20)), count - off);
+        m = std::min(sub, count - off);
         const size_t o_p = m * 32, o_s = a16(o_p + m * pub_sz), o_o = o_s + m * 64;
         uint8_t* h = (uint8_t*)pstage_[j].p;
         uint8_t* d = (uint8_t*)dstage_[j].p;
-        // items [lo, hi) of this chunk into the slot
-        auto pack = [&](size_t lo, size_t hi) {
-            auto one = [&](uint8_t* dst, const uint8_t* src, size_t width, size_t stride) {
+        // One field of this chunk into the slot, then its copy to the device: a
+        // large chunk's next field is packed while the last one is copied.
+        const bool split = m >= kPackSplitItems;
+        size_t copied = 0;
+        auto field = [&](size_t at, const uint8_t* src, size_t width, size_t stride) -> cudaError_t {
+            parallel_copy(m, [&](size_t lo, size_t hi) {
                 if (stride == width) {
-                    memcpy(dst + lo * width, src + (off + lo) * width, (hi - lo) * width);
+                    stage_copy(h + at + lo * width, src + (off + lo) * width, (hi - lo) * width);
                 } else {
-                    for (size_t i = lo; i < hi; ++i) memcpy(dst + i * width, src + (off + i) * stride, width);
+                    stage_rows(h + at + lo * width, src + (off + lo) * stride, width, stride, hi - lo);
                 }
-            };
-            one(h, msgs, 32, m_stride);
-            one(h + o_p, pubs, pub_sz, p_stride);
-            one(h + o_s, sigs, 64, s_stride);
+                stage_fence();
+            });
+            if (!split && at != o_s) return cudaSuccess;
+            size_t end = at + m * width;
+            if (at == o_s && collect) {
+                memcpy(h + o_o, out + off, m);
+                end = o_o + m;
+            }
+            const size_t from = copied;
+            copied = end;
+            return cudaMemcpyAsync(d + from, h + from, end - from, cudaMemcpyHostToDevice, pstream_[j]);
         };
         NvtxRange pack_range("pack chunk");
-        if (pack_threads_ > 1 && m >= kPackSplitItems) {
-            if (!pack_pool_) pack_pool_.reset(new PackPool(pack_threads_));
-            const int parts = pack_pool_->threads();
-            pack_pool_->run(parts, [&](int p) { pack(m * p / parts, m * (p + 1) / parts); });
-        } else {
-            pack(0, m);
-        }
-        if (collect) memcpy(h + o_o, out + off, m);
-        const size_t in_bytes = o_o + (collect ? m : 0);
-        if ((e = cudaMemcpyAsync(d, h, in_bytes, cudaMemcpyHostToDevice, pstream_[j])) != cudaSuccess)
+        if ((e = field(0, msgs, 32, m_stride)) != cudaSuccess || (e = field(o_p, pubs, pub_sz, p_stride)) != cudaSuccess ||
+            (e = field(o_s, sigs, 64, s_stride)) != cudaSuccess)
             return fail(cuda_error(e, "host->device copy"));
-        e = launch_verify(kind, d, d + o_p, d + o_s, (uint32_t)m, d + o_o, collect, pstream_[j], count);
+        // a last chunk of at most half a wave waits for the one before it: its
+        // small blocks would fill the first SMs to finish, two by two
+        if (k > 0 && m <= sub / 2 &&
+            (e = cudaStreamWaitEvent(pstream_[j], pev_[(k - 1) % kPipeSlots], 0)) != cudaSuccess)
+            return fail(cuda_error(e, "event wait"));
+        e = launch_verify(kind, d, d + o_p, d + o_s, (uint32_t)m, d + o_o, collect, pstream_[j]);
         if (e != cudaSuccess) return fail(cuda_error(e, "verify launch"));
         if ((e = cudaMemcpyAsync(h + o_o, d + o_o, m, cudaMemcpyDeviceToHost, pstream_[j])) != cudaSuccess)
             return fail(cuda_error(e, "device->host copy"));
@@ -627,12 +634,18 @@ int Backend::verify_jobs(const VerifyJob* jobs, size_t n_jobs, uint32_t rlc_segm
 }
 
 void Backend::parallel_copy(size_t n, const std::function<void(size_t, size_t)>& fn) {
-    if (pack_threads_ > 1 && n >= kPackSplitItems) {
+    if (n < kPackSplitItems) return fn(0, n);
+    // pieces are taken one at a time: a helper that wakes late takes fewer
+    parallel_run((int)((n + kPackPiece - 1) / kPackPiece),
+                 [&](int p) { fn(p * kPackPiece, std::min(n, (p + 1) * kPackPiece)); });
+}
+
+void Backend::parallel_run(int parts, const std::function<void(int)>& fn) {
+    if (pack_threads_ > 1 && parts > 1) {
         if (!pack_pool_) pack_pool_.reset(new PackPool(pack_threads_));
-        const int parts = pack_pool_->threads();
-        pack_pool_->run(parts, [&](int p) { fn(n * p / parts, n * (p + 1) / parts); });
+        pack_pool_->run(parts, fn);
     } else {
-        fn(0, n);
+        for (int p = 0; p < parts; ++p) fn(p);
     }
 }
 
@@ -648,6 +661,7 @@ int Backend::verify_queue_jobs(const VerifyJob* jobs, size_t n_jobs) {
         if (!batch_[q]) {
             auto slot = std::make_unique<BatchSlot>();
             const int rc = slot->init(this);
+            slot->set_parallel_pack();
             if (rc != kOk) return rc;
             if (keys_) slot->set_cache(keys_->slots(), keys_->mask(), keys_->counters());
             batch_[q] = std::move(slot);
@@ -687,11 +701,9 @@ int Backend::verify_queue_jobs(const VerifyJob* jobs, size_t n_jobs) {
             if ((rc = batch_[q]->finish(part[q].data(), part[q].size())) != kOk) break;
         }
         part[q].clear();
-        // the first sub-calls ramp up from kPipeFirst items, so the device
-        // starts while the CPU packs the next one, to one wave of the verify
-        // kernel's full blocks (256 items per SM: 37,888 on a 148-SM B200)
-        const size_t wave = std::max<size_t>(kPipeFirst, std::min(kJobsPipeItems, (size_t)sms_ * 256));
-        const size_t cap = std::min(wave, kPipeFirst << std::min(k, 8));
+        // one wave of the verify kernel's full blocks (256 items per SM:
+        // 37,888 on a 148-SM B200) per sub-call
+        const size_t cap = std::min(kJobsPipeItems, (size_t)sms_ * 256);
         size_t n = 0;
         while (j < n_jobs && n < cap) {
             const VerifyJob& J = jobs[order[j]];

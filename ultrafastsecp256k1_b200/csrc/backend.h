@@ -181,16 +181,13 @@ private:
     // one; an explicit set_variant / environment override clears it.
     int small_variant_[2] = {-1, -1};
     uint32_t small_items_[2] = {0, 0};
-    // Calls of at most pair_items_[kind] items (kinds 0 and 1) run two lanes
-    // per signature (kernels_pair.cu); 0 = never.  Also cleared by an explicit
-    // variant choice.
+    // Launches of at most pair_items_[kind] items (kinds 0 and 1) run four
+    // warps per 32 signatures (kernels_team.cu); 0 = never.  Also cleared by an
+    // explicit variant choice.
     uint32_t pair_items_[2] = {0, 0};
     int inv_group_[2] = {1, 1};
-    // call_items: the size of the whole call this launch belongs to; the
-    // small-launch variant is used only when the whole call is small (the
-    // chunks of a large call run beside one another at full occupancy).
     cudaError_t launch_verify(int kind, const uint8_t* m, const uint8_t* p, const uint8_t* s, uint32_t n,
-                              uint8_t* out, int collect, cudaStream_t st, size_t call_items);
+                              uint8_t* out, int collect, cudaStream_t st);
     void load_tuning();
     cudaStream_t stream_ = nullptr;
     void* d_gtab_ = nullptr;
@@ -221,6 +218,8 @@ public:
     // fn(lo, hi) over [0, n) split between the staging-copy threads (the
     // caller included) when n is large enough to pay for them.
     void parallel_copy(size_t n, const std::function<void(size_t, size_t)>& fn);
+    // fn(part) for every part in [0, parts) on those threads.
+    void parallel_run(int parts, const std::function<void(int)>& fn);
 
 private:
     uint32_t key_log2_ = 18;

@@ -8,6 +8,7 @@
 
 #include "backend.h"
 #include "nvtx.h"
+#include "stage_copy.h"
 
 namespace uf {
 
@@ -156,6 +157,55 @@ int BatchSlot::run_graph(const QueueArgs& a, uint64_t key) {
     return kOk;
 }
 
+// The jobs' fields into the staging at h, in job order per kind: copies of at
+// most kPackBytes, handed out in runs of about that size.
+void BatchSlot::pack(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, bool parallel) {
+    copies_.clear();
+    runs_.assign(1, 0);
+    size_t run = 0;
+    auto add = [&](uint8_t* dst, const uint8_t* src, size_t bytes) {
+        while (bytes) {
+            const size_t take = std::min(bytes, kPackBytes);
+            copies_.push_back(Copy{dst, src, take});
+            dst += take;
+            src += take;
+            bytes -= take;
+            run += take;
+            if (run >= kPackBytes) {
+                runs_.push_back((uint32_t)copies_.size());
+                run = 0;
+            }
+        }
+    };
+    size_t oe = 0, os = 0;
+    for (size_t j = 0; j < n_jobs; ++j) {
+        const VerifyJob& J = jobs[j];
+        if (J.count == 0) continue;
+        if (J.kind == 0) {
+            add(h + layout_.e_msgs + 32 * oe, J.msgs, 32 * J.count);
+            add(h + layout_.e_sigs + 64 * oe, J.sigs, 64 * J.count);
+            add(h + layout_.e_pubs + 33 * oe, J.pubs, 33 * J.count);
+            oe += J.count;
+        } else {
+            add(h + layout_.s_msgs + 32 * os, J.msgs, 32 * J.count);
+            add(h + layout_.s_sigs + 64 * os, J.sigs, 64 * J.count);
+            add(h + layout_.s_pubs + 32 * os, J.pubs, 32 * J.count);
+            os += J.count;
+        }
+    }
+    if (run) runs_.push_back((uint32_t)copies_.size());
+    auto one = [this](int p) {
+        for (uint32_t c = runs_[p]; c < runs_[p + 1]; ++c) stage_copy(copies_[c].dst, copies_[c].src, copies_[c].bytes);
+        stage_fence();
+    };
+    const int parts = (int)runs_.size() - 1;
+    if (parallel) {
+        be_->parallel_run(parts, one);
+    } else {
+        for (int p = 0; p < parts; ++p) one(p);
+    }
+}
+
 int BatchSlot::enqueue(const VerifyJob* jobs, size_t n_jobs) {
     NvtxRange range("batch slot: pack + launch");
     if (const int rc = be_->fault_point("batch enqueue")) return rc;
@@ -181,22 +231,7 @@ int BatchSlot::enqueue(const VerifyJob* jobs, size_t n_jobs) {
     hdr[0] = (uint32_t)n_e;
     hdr[1] = (uint32_t)n_s;
     hdr[2] = 0;   // the key table's to-do count
-    size_t oe = 0, os = 0;
-    for (size_t j = 0; j < n_jobs; ++j) {
-        const VerifyJob& J = jobs[j];
-        if (J.count == 0) continue;
-        if (J.kind == 0) {
-            memcpy(h + layout_.e_msgs + 32 * oe, J.msgs, 32 * J.count);
-            memcpy(h + layout_.e_sigs + 64 * oe, J.sigs, 64 * J.count);
-            memcpy(h + layout_.e_pubs + 33 * oe, J.pubs, 33 * J.count);
-            oe += J.count;
-        } else {
-            memcpy(h + layout_.s_msgs + 32 * os, J.msgs, 32 * J.count);
-            memcpy(h + layout_.s_sigs + 64 * os, J.sigs, 64 * J.count);
-            memcpy(h + layout_.s_pubs + 32 * os, J.pubs, 32 * J.count);
-            os += J.count;
-        }
-    }
+    pack(jobs, n_jobs, h, parallel_pack_ && n_e + n_s >= kParallelPackItems);
     uint8_t* d = staged_big_ ? (uint8_t*)big_dev_.p : (uint8_t*)dev_.p;
     const QueueArgs a = args_for(d);
     last_graph_ = graph;

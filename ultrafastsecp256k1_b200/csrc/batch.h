@@ -65,12 +65,24 @@ public:
         cache_mask_ = mask;
         cache_stats_ = stats;
     }
+    // Large launches' staging is packed by the backend's pool as well as the
+    // caller (slots that only the backend's calling thread uses).
+    void set_parallel_pack() { parallel_pack_ = true; }
     cudaStream_t stream() const { return stream_; }
     size_t staged_bytes() const { return layout_.total; }
     size_t graphs_cached() const { return graphs_.size(); }
     bool last_used_graph() const { return last_graph_; }
 
 private:
+    static constexpr size_t kParallelPackItems = size_t{1} << 13;
+    static constexpr size_t kPackBytes = size_t{1} << 16;
+    struct Copy {
+        uint8_t* dst;
+        const uint8_t* src;
+        size_t bytes;
+    };
+
+    void pack(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, bool parallel);
     int run_direct(const QueueArgs& a);
     bool small_launch(const QueueArgs& a) const;
     uint64_t graph_key(const QueueArgs& a) const;
@@ -91,6 +103,9 @@ private:
     QueueLayout layout_;
     bool staged_big_ = false;
     bool last_graph_ = false;
+    bool parallel_pack_ = false;
+    std::vector<Copy> copies_;       // the launch's staging copies, runs_[p] .. runs_[p + 1] one part
+    std::vector<uint32_t> runs_;
     std::map<uint64_t, cudaGraphExec_t> graphs_;
     PubCacheSlot* cache_ = nullptr;
     uint32_t cache_mask_ = 0;
