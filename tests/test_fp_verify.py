@@ -279,6 +279,23 @@ def test_chunks_and_last_waves(plain_ctx, oracle, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [37889, 47361, 56832, 56833])
+def test_device_last_waves(plain_ctx, oracle, n):
+    import torch
+    m, p, s = schnorr_corpus(oracle, 701, 18, tamper=0.1)
+    order = np.random.default_rng(n).integers(0, 701, n)
+    want = oracle.schnorr_verify_batch(m, p, s)[order]
+    d = [torch.from_numpy(np.ascontiguousarray(a[order])).cuda() for a in (m, p, s)]
+    out = torch.full((n + 1,), 7, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    plain_ctx.schnorr_verify_device(*(a.data_ptr() for a in d), n, out.data_ptr(), stream=stream.cuda_stream)
+    stream.synchronize()
+    got = out.cpu().numpy()
+    assert (got[:n] == want).all() and got[n] == 7
+
+
+@pytest.mark.gpu
 def test_jobs_packed_in_pieces(plain_ctx, oracle):
     em, ep, es = ecdsa_corpus(oracle, 701, 17)
     sm, sp, ss = schnorr_corpus(oracle, 701, 18, tamper=0.1)
