@@ -46,8 +46,9 @@ public:
     // Creates the stream, completion event and queue head on the backend's device.
     int init(Backend* be, bool use_graphs = true);
     // Packs `jobs` and enqueues the work; returns immediately.  The jobs' host
-    // buffers must stay valid until finish() returns.
-    int enqueue(const VerifyJob* jobs, size_t n_jobs);
+    // buffers must stay valid until finish() returns.  in_flight: items that
+    // other slots have on the device at that time.
+    int enqueue(const VerifyJob* jobs, size_t n_jobs, size_t in_flight = 0);
     // Captures and runs (with zero items) the graph of every capacity bucket
     // pair whose total is at most max_items, so that later launches of any
     // shape find their graph instantiated and their kernels loaded.
@@ -104,6 +105,7 @@ private:
     bool staged_big_ = false;
     bool last_graph_ = false;
     bool parallel_pack_ = false;
+    uint64_t beside_ = 0;            // items on the device with this launch beside other slots' (0: alone)
     std::vector<Copy> copies_;       // the launch's staging copies, runs_[p] .. runs_[p + 1] one part
     std::vector<uint32_t> runs_;
     std::map<uint64_t, cudaGraphExec_t> graphs_;

@@ -264,9 +264,12 @@ void Server::loop() {
                     std::chrono::duration<double, std::micro>(Clock::now() - pending_.front()->t_submit).count();
                 if (queued < cfg_.max_launch_items / 4 && age_us < cfg_.batch_window_us) break;
             }
+            size_t in_flight = 0;
+            for (const Launch& O : launches_)
+                for (const VerifyJob& J : O.jobs) in_flight += J.count;
             if (!admit(L)) break;
             lk.unlock();
-            const int rc = L.slot->enqueue(L.jobs.data(), L.jobs.size());
+            const int rc = L.slot->enqueue(L.jobs.data(), L.jobs.size(), in_flight);
             lk.lock();
             if (rc != kOk) complete(L, rc);
             progressed = true;
