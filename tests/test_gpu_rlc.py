@@ -378,3 +378,21 @@ def test_rlc_uses_resident_keys(oracle):
         ctx.set_key_table(0)
         out2, _ = ctx.schnorr_verify_rlc(m, x, s, batch_size=512, seed32=SEED)
         assert (out2 == want).all() and ctx.rlc_stats()["key_hits"] == 0
+
+
+@pytest.mark.parametrize("batch,wbits", [(1, 4), (2, 5), (3, 4), (9, 6), (40, 8), (700, 9), (1400, 11), (2800, 13)])
+def test_rlc_shapes_of_the_window_sums(gpu_ctx, oracle, batch, wbits):
+    """1 to 2,800 segments with 4- to 13-bit windows: 2 to 256 lanes per window
+    sum, 1 to 32 per Horner chain; equal points in one bucket and a cancelling
+    bad item among them."""
+    m, x, s = schnorr_corpus(oracle, 90, seed=84, tamper=0.0)
+    _flip(m, 7)
+    rng = np.random.default_rng(batch)
+    idx = rng.integers(8, 90, 2800)
+    idx[rng.choice(2800, 3, replace=False)] = 7
+    m, x, s = m[idx].copy(), x[idx].copy(), s[idx].copy()
+    want = (idx != 7).astype(np.uint8)
+    assert (oracle.schnorr_verify_batch(m, x, s) == want).all()
+    out, bok = gpu_ctx.schnorr_verify_rlc(m, x, s, batch_size=batch, seed32=SEED, window_bits=wbits)
+    assert (out == want).all()
+    assert bok.tolist() == [int(want[i:i + batch].all()) for i in range(0, 2800, batch)]

@@ -108,6 +108,7 @@ public:
     // items: the fixed override if set, else the value of the nearest tuned
     // batch size (tuning file lines "rlc_chunk_<n> <points>"), else 16.
     uint32_t rlc_chunk(uint32_t len) const;
+    bool rlc_chunk_fixed() const { return rlc_chunk_fixed_ != 0; }
     // 2..256 fixes the chunk for every segment length; 0 restores the tuned values.
     int set_rlc_chunk(uint32_t chunk);
     // Whether a failing RLC segment first gets a locate round (one more MSM

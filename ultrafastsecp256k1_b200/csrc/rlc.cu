@@ -5,8 +5,8 @@
 // c-bit windows (W = ceil(129 / c) windows, B = 2^(c-1) buckets per window):
 // one 4-byte entry per non-zero digit (at most (3 len + 2) W per segment),
 // counters and offsets over the K = S W B bucket keys, a Jacobian sum (112 B)
-// per bucket and per chunk of chunk() entries, two per bucket sub-range and one
-// per window.
+// per bucket, per chunk of at most chunk() entries and per window, and a 16-byte
+// record per chunk.
 #include "rlc.h"
 
 #include <string.h>
@@ -40,12 +40,15 @@ struct RlcSeed {
     uint8_t b[32];
 };
 
-// Running sums of a window's B buckets are split into S sub-ranges of B / S
-// buckets (one thread each) and the S partial results joined by a tree over S
-// lanes, at most a warp.  Narrow windows (c <= 8) come with many segments, which
-// fill the device: S = 2^floor((c - 1) / 2); for wider ones the chain of B / S
-// additions is what counts: S = 32.
-inline int sub_ranges(int c) { return c >= 9 ? 32 : 1 << ((c - 1) / 2); }
+// Lanes per window sum (a power of two), each over B / S buckets: about the
+// square root of B where the windows fill the device, more (up to 256, down to
+// four buckets a lane) while twice as many still leave it at two warps per
+// scheduler.
+inline int window_lanes(int c, uint64_t windows) {
+    int S = c >= 9 ? 32 : 1 << ((c - 1) / 2);
+    while (S < 256 && 8 * S <= 1 << (c - 1) && 2 * S * windows <= 2 * 592 * 32) S *= 2;
+    return S;
+}
 
 // Signed digit of window w (c bits) of a magnitude m + hi 2^128 < 2^160 (the
 // recoding of booth_recode in ecmult.cuh with a run-time window width).
@@ -288,41 +291,110 @@ k_rlc_digits(RoundGeo g, const uint4* __restrict__ mags, const uint32_t* __restr
     }
 }
 
-// chunks per key, for the chunk scan; nch[K] = 0
-__global__ void k_rlc_nchunks(const uint32_t* __restrict__ counts, uint32_t K, uint32_t chunk,
-                              uint32_t* __restrict__ nch) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < K) nch[k] = (counts[k] + chunk - 1) / chunk;
-    else if (k == K) nch[k] = 0;
+// A bucket of c entries is cut into ceil(c / chunk) chunks of nearly equal
+// length, and the chunks are listed by length, longest first (a counting sort
+// over the at most kRlcMaxChunk + 1 lengths), so that the threads of a warp sum
+// chunks of one length: in bucket order with chunks of 12, a warp of 4,096-item
+// batches (24 entries a bucket) waited for its longest chunk a quarter of the time.
+constexpr int kRlcMaxChunk = 256;
+
+struct ChunkCut {
+    uint32_t n, len, longer;     // n chunks, `longer` of them of len + 1 entries, the others of len
+};
+
+__device__ __forceinline__ ChunkCut chunk_cut(uint32_t count, uint32_t chunk) {
+    ChunkCut c;
+    c.n = (count + chunk - 1) / chunk;
+    c.len = c.n ? count / c.n : 0;
+    c.longer = c.n ? count % c.n : 0;
+    return c;
 }
 
-// The bucket key of every chunk.
+// Chunks per key, for the chunk scan (nch[K] = 0), and chunks per length in
+// bins[0 .. kRlcMaxChunk] (zeroed before).
 __global__ void __launch_bounds__(256)
-k_rlc_chunk_keys(const uint32_t* __restrict__ coff, uint32_t K, uint32_t* __restrict__ ckey) {
+k_rlc_nchunks(const uint32_t* __restrict__ counts, uint32_t K, uint32_t chunk, uint32_t* __restrict__ nch,
+              uint32_t* __restrict__ bins) {
+    __shared__ uint32_t bin[kRlcMaxChunk + 1];
+    for (int b = threadIdx.x; b <= kRlcMaxChunk; b += blockDim.x) bin[b] = 0;
+    __syncthreads();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    for (uint32_t t = coff[k]; t < coff[k + 1]; ++t) ckey[t] = k;
+    if (k < K) {
+        const ChunkCut c = chunk_cut(counts[k], chunk);
+        nch[k] = c.n;
+        if (c.longer) atomicAdd(&bin[c.len + 1], c.longer);
+        if (c.n > c.longer) atomicAdd(&bin[c.len], c.n - c.longer);
+    } else if (k == K) {
+        nch[k] = 0;
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b <= kRlcMaxChunk; b += blockDim.x)
+        if (bin[b]) atomicAdd(&bins[b], bin[b]);
 }
 
-// One thread per chunk of at most `chunk` entries of one bucket, summed by
-// mixed additions on the FP64 pipe (XYZZ form: 3.8 k cycles each per warp and
-// scheduler, the register-read bound of fd.cuh).  A bucket with a single chunk
-// is written straight to its bucket slot.  It replaced pairwise trees of affine
-// additions whose inversions were shared by the grid (5M + 1S each, but every
-// level went through memory): 64 batches of 4,096 1.95 -> 1.26 ms a round.
+// bins[b] = chunks longer than b: where length b starts in the list.
+__global__ void __launch_bounds__(512) k_rlc_bins(uint32_t* __restrict__ bins) {
+    __shared__ uint32_t sum[512];
+    const int t = threadIdx.x, b = kRlcMaxChunk - t;
+    const uint32_t own = b >= 0 ? bins[b] : 0;
+    sum[t] = own;
+    for (int d = 1; d < 512; d <<= 1) {
+        __syncthreads();
+        const uint32_t below = t >= d ? sum[t - d] : 0;
+        __syncthreads();
+        sum[t] += below;
+    }
+    if (b >= 0) bins[b] = sum[t] - own;
+}
+
+// The list: {key, first entry, length, chunk index or kSingleChunk}.
+constexpr uint32_t kSingleChunk = 0xFFFFFFFFu;
+
+__global__ void __launch_bounds__(256)
+k_rlc_chunk_list(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ offsets,
+                 const uint32_t* __restrict__ coff, uint32_t K, uint32_t chunk, uint32_t* __restrict__ bins,
+                 uint4* __restrict__ list) {
+    __shared__ uint32_t bin[kRlcMaxChunk + 1];
+    for (int b = threadIdx.x; b <= kRlcMaxChunk; b += blockDim.x) bin[b] = 0;
+    __syncthreads();
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    ChunkCut c = {0, 0, 0};
+    uint32_t at_longer = 0, at_len = 0;
+    if (k < K) c = chunk_cut(counts[k], chunk);
+    if (c.longer) at_longer = atomicAdd(&bin[c.len + 1], c.longer);
+    if (c.n > c.longer) at_len = atomicAdd(&bin[c.len], c.n - c.longer);
+    __syncthreads();
+    for (int b = threadIdx.x; b <= kRlcMaxChunk; b += blockDim.x)
+        if (bin[b]) bin[b] = atomicAdd(&bins[b], bin[b]);
+    __syncthreads();
+    if (c.n == 0) return;
+    if (c.longer) at_longer += bin[c.len + 1];
+    at_len += bin[c.len];
+    uint32_t e = offsets[k];
+    for (uint32_t i = 0; i < c.n; ++i) {
+        const bool more = i < c.longer;
+        const uint32_t len = c.len + (more ? 1u : 0u);
+        list[more ? at_longer++ : at_len++] = make_uint4(k, e, len, c.n == 1 ? kSingleChunk : coff[k] + i);
+        e += len;
+    }
+}
+
+// One thread per chunk of entries of one bucket, summed by mixed additions on the
+// FP64 pipe (XYZZ form: 3.9 k cycles each per warp and scheduler, the
+// register-read bound of fd.cuh).  A bucket with a single chunk is written
+// straight to its bucket slot.  It replaced pairwise trees of affine additions
+// whose inversions were shared by the grid (5M + 1S each, but every level went
+// through memory): 64 batches of 4,096 1.95 -> 1.09 ms a round.
 constexpr int kChunkThreads = 128;
 
 __global__ void __launch_bounds__(kChunkThreads, 2)
-k_rlc_chunks(const uint32_t* __restrict__ coff, uint32_t K, uint32_t chunk, const uint32_t* __restrict__ offsets,
-             const uint32_t* __restrict__ entries, const uint32_t* __restrict__ ckey,
-             const RlcItem* __restrict__ items, uint32_t n3, const uint4* __restrict__ gt,
-             uint4* __restrict__ partials, uint4* __restrict__ buckets) {
+k_rlc_chunks(const uint32_t* __restrict__ coff, uint32_t K, const uint4* __restrict__ list,
+             const uint32_t* __restrict__ entries, const RlcItem* __restrict__ items, uint32_t n3,
+             const uint4* __restrict__ gt, uint4* __restrict__ partials, uint4* __restrict__ buckets) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= coff[K]) return;
-    const uint32_t key = ckey[t];
-    const uint32_t j = t - coff[key];
-    const uint32_t e0 = offsets[key] + j * chunk;
-    const uint32_t e1 = min(e0 + chunk, offsets[key + 1]);
+    const uint4 rec = list[t];
+    const uint32_t e0 = rec.y, e1 = rec.y + rec.z;
     XyzzD acc;
     xyzzd_set_inf(acc);
     // the next entry's point is fetched while this one is added
@@ -346,8 +418,8 @@ k_rlc_chunks(const uint32_t* __restrict__ coff, uint32_t K, uint32_t chunk, cons
         xyzzd_add_aff(acc, x, y);
     }
     const JacD sum = xyzzd_to_jac(acc);
-    if (coff[key + 1] - coff[key] == 1) store_jacd(buckets + kJacQ * (uint64_t)key, sum);
-    else store_jacd(partials + kJacQ * (uint64_t)t, sum);
+    if (rec.w == kSingleChunk) store_jacd(buckets + kJacQ * (uint64_t)rec.x, sum);
+    else store_jacd(partials + kJacQ * (uint64_t)rec.w, sum);
 }
 
 // ---------------------------------------------------------------- locate --
@@ -683,10 +755,10 @@ int rlc_window_bits(uint32_t len) {
 
 RlcVerifier::~RlcVerifier() {
     for (DevBuf* b : {&items_, &mags_, &tsc_, &okb_, &segs_, &segmag_, &segneg_, &segbad_, &counts_, &offsets_,
-                      &cursor_, &nch_, &coff_, &entries_, &partials_, &buckets_, &wu_, &wt_, &wins_, &segok_,
+                      &cursor_, &nch_, &coff_, &entries_, &partials_, &buckets_, &wins_, &segok_,
                       &scan_tmp_, &leaf_idx_, &leaf_m_, &leaf_x_, &leaf_s_, &leaf_out_, &in_m_, &in_x_, &in_s_,
                       &in_out_, &in_rows_, &gate_, &segpt_, &dig_a_, &dig_b_, &lmags_, &lmags_hi_, &tsave_,
-                      &loc_idx_, &found_, &heavy_, &ckey_, &keyhit_})
+                      &loc_idx_, &found_, &heavy_, &crec_, &bins_, &keyhit_})
         b->release();
     job_host_.release();
 }
@@ -703,7 +775,7 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     int mag_bits = 129;
     if (locate)
         for (uint32_t v = maxlen; v; v >>= 1) ++mag_bits;
-    const int W = (mag_bits + c - 1) / c, B = 1 << (c - 1), S = sub_ranges(c);
+    const int W = (mag_bits + c - 1) / c, B = 1 << (c - 1), S = window_lanes(c, (uint64_t)n_seg * W);
     std::vector<uint32_t> host(3 * (size_t)n_seg + 1);
     uint64_t total = 0;
     for (uint32_t k = 0; k < n_seg; ++k) {
@@ -716,7 +788,12 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     host[3 * (size_t)n_seg] = (uint32_t)total;
     const uint64_t K = (uint64_t)n_seg * W * B;
     if (K >= 0x7FFFFFFFull) return be_->set_error(kErrBadInput, "RLC round too large");
-    const uint32_t chunk = be_->rlc_chunk(maxlen);
+    // A round of few entries is cut finer than tuned, to about two chunks per
+    // thread of the device: 8,192 items in one batch 2.0 ms with chunks of 96,
+    // 1.7 with 24; 262,144 at 4,096 per batch 4.6 with 8, 4.3 with 48 - 96.
+    uint32_t chunk = be_->rlc_chunk(maxlen);
+    if (!be_->rlc_chunk_fixed())
+        chunk = std::min(chunk, std::max(24u, (uint32_t)(total / ((uint64_t)be_->sms() * 256))));
     const uint64_t chunk_cap = total / chunk + K + 1;
     size_t scan_bytes = 0;
     cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
@@ -727,11 +804,10 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
         (e = counts_.ensure((K + 1) * 4)) != cudaSuccess || (e = offsets_.ensure((K + 1) * 4)) != cudaSuccess ||
         (e = cursor_.ensure(std::max<uint64_t>(total, 1) * 4)) != cudaSuccess ||
         (e = nch_.ensure((K + 1) * 4)) != cudaSuccess ||
-        (e = coff_.ensure((K + 1) * 4)) != cudaSuccess || (e = ckey_.ensure(chunk_cap * 4)) != cudaSuccess ||
+        (e = coff_.ensure((K + 1) * 4)) != cudaSuccess || (e = crec_.ensure(chunk_cap * 16)) != cudaSuccess ||
+        (e = bins_.ensure((kRlcMaxChunk + 1) * 4)) != cudaSuccess ||
         (e = entries_.ensure(std::max<uint64_t>(total, 1) * 4)) != cudaSuccess ||
         (e = partials_.ensure(chunk_cap * 112)) != cudaSuccess || (e = buckets_.ensure(K * 112)) != cudaSuccess ||
-        (e = wu_.ensure((uint64_t)n_seg * W * S * 112)) != cudaSuccess ||
-        (e = wt_.ensure((uint64_t)n_seg * W * S * 112)) != cudaSuccess ||
         (e = wins_.ensure((uint64_t)n_seg * W * 112)) != cudaSuccess || (e = segok_.ensure(n_seg)) != cudaSuccess ||
         (e = segpt_.ensure((uint64_t)n_seg * 112)) != cudaSuccess ||
         // a heavy bucket holds more than kHeavyChunks of the at most chunk_cap chunks
@@ -752,6 +828,7 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     e = cudaMemcpyAsync(d_seg, host.data(), host.size() * 4, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, (K + 1) * 4, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(heavy_.p, 0, 4, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(bins_.p, 0, (kRlcMaxChunk + 1) * 4, s);
     if (e != cudaSuccess) return be_->cuda_error(e, "RLC round set-up");
     if (locate)
         k_rlc_scale<<<dim3(n_seg, (maxlen + 255) / 256), 256, 0, s>>>(d_seg, (const uint4*)mags_.p,
@@ -769,19 +846,22 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     k_rlc_digits<<<grid_for(total / (size_t)W, 256), 256, 0, s>>>(g, mags, mags_hi, (const uint4*)segmag_.p,
                                                                  (const uint8_t*)segneg_.p, (uint32_t)total, nullptr,
                                                                  ranks, offsets, (uint32_t*)entries_.p, 1);
-    k_rlc_nchunks<<<grid_for(K + 1, 256), 256, 0, s>>>(counts, (uint32_t)K, chunk, nch);
+    uint32_t* bins = (uint32_t*)bins_.p;
+    k_rlc_nchunks<<<grid_for(K + 1, 256), 256, 0, s>>>(counts, (uint32_t)K, chunk, nch, bins);
+    k_rlc_bins<<<1, 512, 0, s>>>(bins);
     tb = scan_tmp_.cap;
     e = cub::DeviceScan::ExclusiveSum(scan_tmp_.p, tb, nch, coff, (int)(K + 1), s);
     if (e != cudaSuccess) return be_->cuda_error(e, "RLC chunk scan");
-    k_rlc_chunk_keys<<<grid_for(K, 256), 256, 0, s>>>(coff, (uint32_t)K, (uint32_t*)ckey_.p);
+    k_rlc_chunk_list<<<grid_for(K, 256), 256, 0, s>>>(counts, offsets, coff, (uint32_t)K, chunk, bins,
+                                                      (uint4*)crec_.p);
     k_rlc_chunks<<<grid_for(chunk_cap, kChunkThreads), kChunkThreads, 0, s>>>(
-        coff, (uint32_t)K, chunk, offsets, (const uint32_t*)entries_.p, (const uint32_t*)ckey_.p,
-        (const RlcItem*)items_.p, 3u * n_, (const uint4*)be_->gtab(), (uint4*)partials_.p, (uint4*)buckets_.p);
+        coff, (uint32_t)K, (const uint4*)crec_.p, (const uint32_t*)entries_.p, (const RlcItem*)items_.p, 3u * n_,
+        (const uint4*)be_->gtab(), (uint4*)partials_.p, (uint4*)buckets_.p);
     e = launch_rlc_bucket_merge(coff, (uint32_t)K, (const uint4*)partials_.p, (uint4*)buckets_.p,
                                 (uint32_t*)heavy_.p, be_->sms() * 4, s);
     if (e != cudaSuccess) return be_->cuda_error(e, "RLC bucket merge");
-    e = launch_rlc_windows(g, (const uint4*)buckets_.p, (uint4*)wu_.p, (uint4*)wt_.p, (uint4*)wins_.p,
-                           (const uint32_t*)segbad_.p, (uint8_t*)segok_.p, (uint4*)segpt_.p, s);
+    e = launch_rlc_windows(g, (const uint4*)buckets_.p, (uint4*)wins_.p, (const uint32_t*)segbad_.p,
+                           (uint8_t*)segok_.p, (uint4*)segpt_.p, s);
     if (e == cudaSuccess) e = cudaGetLastError();
     ok.resize(n_seg);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ok.data(), segok_.p, n_seg, cudaMemcpyDeviceToHost, s);

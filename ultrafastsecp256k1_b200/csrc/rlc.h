@@ -144,7 +144,7 @@ private:
     // per round
     // cursor_: each entry's rank in its bucket (k_rlc_digits)
     DevBuf segs_, segmag_, segneg_, segbad_, counts_, offsets_, cursor_, nch_, coff_, entries_, partials_,
-        buckets_, wu_, wt_, wins_, segok_, scan_tmp_;
+        buckets_, wins_, segok_, scan_tmp_;
     // leaves
     DevBuf leaf_idx_, leaf_m_, leaf_x_, leaf_s_, leaf_out_;
     // host-buffer calls
@@ -153,7 +153,7 @@ private:
     DevBuf dig_a_, dig_b_;   // input digest tree levels
     DevBuf lmags_, lmags_hi_, tsave_, loc_idx_, found_;   // locate step
     DevBuf heavy_;       // count and keys of the buckets with many chunks (k_rlc_bucket_heavy)
-    DevBuf ckey_;                                           // bucket key of every chunk
+    DevBuf crec_, bins_;                                    // chunk records, their counts by length
     HostBuf job_host_;   // pinned staging of the staged jobs
     DevBuf keyhit_;      // key-table hits of the prep pass
     std::vector<VerifyJob> part_;   // the staged job pieces, and their first items

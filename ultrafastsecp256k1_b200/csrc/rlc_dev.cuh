@@ -83,7 +83,7 @@ struct RoundGeo {
 };
 
 // A bucket of more than this many chunks is merged by a warp (k_rlc_bucket_heavy).
-constexpr uint32_t kHeavyChunks = 48;
+constexpr uint32_t kHeavyChunks = 8;
 
 }  // namespace rlcdev
 }  // namespace uf

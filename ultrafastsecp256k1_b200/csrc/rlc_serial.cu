@@ -1,12 +1,10 @@
 // The RLC kernels with one serial chain per bucket, segment or window: the
-// merge of a bucket's chunk sums, the running sums, the window combination and
-// Horner.  All but the merge run a few thousand threads at most, so a chain's
+// merge of a bucket's chunk sums, the window sums and Horner.  All but the merge run a few thousand threads at most, so a chain's
 // latency, not the issue rate, sets their time: they use the FP64 field
 // arithmetic (fd.cuh), whose products are independent where the limb form is a
 // chain of carries (a doubling alone on its scheduler 2.3 k cycles against
-// 5.0 k), as many sub-ranges as a warp has lanes, and a tree instead of a chain
-// to combine them.  64 segments of 4,096 items, window 10, per round: running
-// sums 365 -> 232 us, combination 288 -> 216 us, Horner 368 -> 214 us.
+// 5.0 k), and trees over a warp's lanes instead of chains.  64 segments of 4,096
+// items, window 10: window sums 653 -> 329 us, Horner 368 -> 155 us.
 #include "rlc_serial.h"
 
 #include "jacd.cuh"
@@ -35,74 +33,100 @@ __device__ __forceinline__ JacD shfl_jacd(const JacD& a, int src) {
     return b;
 }
 
-// One thread per (segment, window, sub-range j of m buckets):
-// T_j = sum_b bucket_b, U_j = sum_b (b - j m + 1) bucket_b by running sums.
-__global__ void __launch_bounds__(128)
-k_rlc_wpart(RoundGeo g, const uint4* __restrict__ buckets, uint4* __restrict__ wu, uint4* __restrict__ wt) {
+// Window sums: S lanes per (segment, window), lane j over m = B / S buckets.
+//   T_j = sum_b bucket_b, U_j = sum_b (b - j m + 1) bucket_b by running sums,
+//   window = sum_j U_j + m sum_j j T_j,  sum_j j T_j = sum_(j >= 1) T'_j
+// with the suffix sums T'_j = T_j + T_(j+1) + ...: a scan, log2(m) doublings of
+// every lane's T'_j at once, and a tree.  (A tree over (U, T) pairs alone doubles
+// T by each range's length: 30 doublings and 10 additions where this takes 4 and
+// 11 for m = 16.)  Blocks are one warp, or the S / 32 warps of one window.
+__global__ void __launch_bounds__(256)
+k_rlc_window(RoundGeo g, const uint4* __restrict__ buckets, uint4* __restrict__ wins) {
+    __shared__ JacD part[8];
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= g.n_seg * (uint32_t)(g.W * g.S)) return;
     const uint32_t sw = q / (uint32_t)g.S, j = q - sw * (uint32_t)g.S;
+    const bool live = sw < g.n_seg * (uint32_t)g.W;
+    const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5), warps = (int)(blockDim.x >> 5);
+    const int width = g.S < 32 ? g.S : 32, at = lane & (width - 1);     // this window's lanes of the warp
     const int m = g.B / g.S;
-    const uint4* base = buckets + kJacQ * ((uint64_t)sw * g.B + (uint64_t)j * m);
     JacD run, tot, b;
     jacd_set_inf(run);
     jacd_set_inf(tot);
-    for (int k = m - 1; k >= 0; --k) {
-        load_jacd(base + kJacQ * k, b);
-        run = jacd_add(run, b);
-        tot = jacd_add(tot, run);
+    if (live) {
+        const uint4* base = buckets + kJacQ * ((uint64_t)sw * g.B + (uint64_t)j * m);
+        for (int k = m - 1; k >= 0; --k) {
+            load_jacd(base + kJacQ * k, b);
+            run = jacd_add(run, b);
+            tot = jacd_add(tot, run);
+        }
     }
-    store_jacd(wu + kJacQ * (uint64_t)q, tot);
-    store_jacd(wt + kJacQ * (uint64_t)q, run);
+    __syncwarp();
+    for (int d = 1; d < width; d <<= 1) {
+        const JacD o = shfl_jacd(run, at + d < width ? lane + d : lane);
+        if (at + d < width) run = jacd_add(run, o);
+        __syncwarp();
+    }
+    if (warps > 1) {
+        if (lane == 0) part[warp] = run;
+        __syncthreads();
+        JacD above;
+        jacd_set_inf(above);
+        for (int v = warps - 1; v > warp; --v) above = jacd_add(above, part[v]);
+        run = jacd_add(run, above);
+        __syncthreads();
+    }
+    int log2m = 0;
+    while (m >> (log2m + 1)) ++log2m;
+    if (j == 0) jacd_set_inf(run);
+    tot = jacd_add(tot, jacd_dbl_n(run, log2m));
+    __syncwarp();
+    for (int d = 1; d < width; d <<= 1) {
+        const JacD o = shfl_jacd(tot, at + d < width ? lane + d : lane);
+        if (at + d < width) tot = jacd_add(tot, o);
+        __syncwarp();
+    }
+    if (warps > 1) {
+        if (lane == 0) part[warp] = tot;
+        __syncthreads();
+        for (int v = 1; threadIdx.x == 0 && v < warps; ++v) tot = jacd_add(tot, part[v]);
+    }
+    if (live && j == 0) store_jacd(wins + kJacQ * (uint64_t)sw, tot);
 }
 
-// S lanes per (segment, window), a power of two of at most 32: window sum =
-// sum_j U_j + m sum_j j T_j by a tree over neighbouring ranges.  A range of
-// 2^k sub-ranges keeps T = sum of its T_j and U = its sum of (bucket - first
-// bucket + 1) weights, so two neighbours join as U + U' + m 2^k T', T + T'.
-__global__ void __launch_bounds__(128)
-k_rlc_wcomb(RoundGeo g, const uint4* __restrict__ wu, const uint4* __restrict__ wt, uint4* __restrict__ wins) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t total = g.n_seg * (uint32_t)(g.W * g.S);
-    const int lane = (int)(threadIdx.x & 31u);
-    JacD U, T;
-    jacd_set_inf(U);
-    jacd_set_inf(T);
-    if (q < total) {
-        load_jacd(wu + kJacQ * (uint64_t)q, U);
-        load_jacd(wt + kJacQ * (uint64_t)q, T);
-    }
-    int log2len = 0;
-    while ((g.B / g.S) >> (log2len + 1)) ++log2len;            // m = B / S
-    for (int d = 1; d < g.S; d <<= 1, ++log2len) {
-        // lanes that are not a range's first compute along and are not used
-        const int src = lane + d < 32 ? lane + d : lane;
-        const JacD U2 = shfl_jacd(U, src);
-        const JacD T2 = shfl_jacd(T, src);
-        U = jacd_add(U, U2);
-        U = jacd_add(U, jacd_dbl_n(T2, log2len));
-        if (2 * d < g.S) T = jacd_add(T, T2);
-    }
-    if (q < total && q % (uint32_t)g.S == 0) store_jacd(wins + kJacQ * (uint64_t)(q / (uint32_t)g.S), U);
-}
-
-// One thread per segment: Horner over the windows; ok = 1 if the sum is
-// infinity, | 2 if the segment holds an item that failed to parse.
+// Horner over the windows, `lanes` (a power of two of at most 32) per segment: a
+// lane takes ceil(W / lanes) neighbouring windows by Horner's rule, doubles the
+// result up to its place, all lanes at once, and a tree adds them: the chain
+// keeps its 129 doublings but has about W / lanes + log2(lanes) additions instead
+// of W - 1.  ok = 1 if the sum is infinity, | 2 if the segment holds an item that
+// failed to parse.
 __global__ void __launch_bounds__(32)
-k_rlc_finish(RoundGeo g, const uint4* __restrict__ wins, const uint32_t* __restrict__ segbad,
+k_rlc_finish(RoundGeo g, int lanes, const uint4* __restrict__ wins, const uint32_t* __restrict__ segbad,
              uint8_t* __restrict__ segok, uint4* __restrict__ segpt) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= g.n_seg) return;
-    const uint4* base = wins + kJacQ * (uint64_t)s * g.W;
+    const uint32_t q = blockIdx.x * 32 + threadIdx.x, s = q / (uint32_t)lanes;
+    const int lane = (int)threadIdx.x, at = lane & (lanes - 1);
+    const int per = (g.W + lanes - 1) / lanes, first = at * per, last = first + per < g.W ? first + per : g.W;
     JacD acc, w;
-    load_jacd(base + kJacQ * (g.W - 1), acc);
-    for (int k = g.W - 2; k >= 0; --k) {
-        acc = jacd_dbl_n(acc, g.c);
-        load_jacd(base + kJacQ * k, w);
-        acc = jacd_add(acc, w);
+    jacd_set_inf(acc);
+    if (s < g.n_seg && first < last) {
+        const uint4* base = wins + kJacQ * (uint64_t)s * g.W;
+        load_jacd(base + kJacQ * (last - 1), acc);
+        for (int k = last - 2; k >= first; --k) {
+            acc = jacd_dbl_n(acc, g.c);
+            load_jacd(base + kJacQ * k, w);
+            acc = jacd_add(acc, w);
+        }
+        acc = jacd_dbl_n(acc, g.c * first);
     }
-    segok[s] = (uint8_t)((acc.inf ? 1 : 0) | (segbad[s] ? 2 : 0));
-    store_jacd(segpt + kJacQ * (uint64_t)s, acc);
+    __syncwarp();
+    for (int d = 1; d < lanes; d <<= 1) {
+        const JacD o = shfl_jacd(acc, at + d < lanes ? lane + d : lane);
+        if (at + d < lanes) acc = jacd_add(acc, o);
+        __syncwarp();
+    }
+    if (s < g.n_seg && at == 0) {
+        segok[s] = (uint8_t)((acc.inf ? 1 : 0) | (segbad[s] ? 2 : 0));
+        store_jacd(segpt + kJacQ * (uint64_t)s, acc);
+    }
 }
 
 // Buckets with 0 or >= 2 chunks: infinity, or the sum of their partials.
@@ -154,47 +178,18 @@ k_rlc_bucket_heavy(const uint32_t* __restrict__ coff, const uint4* __restrict__ 
     }
 }
 
-constexpr uint64_t kWarpHornerSegments = 592;      // one warp per scheduler of a 148-SM device
-
-// The same with a warp per segment (at most 32 windows): lane w doubles window
-// w's sum c w times, all windows at once, and a tree adds them: the chain has the
-// same doublings but log2(W) additions instead of W - 1.  For rounds of few
-// segments; many fill the device with a thread each.
-__global__ void __launch_bounds__(32)
-k_rlc_finish_warp(RoundGeo g, const uint4* __restrict__ wins, const uint32_t* __restrict__ segbad,
-                  uint8_t* __restrict__ segok, uint4* __restrict__ segpt) {
-    const uint32_t s = blockIdx.x;
-    const int lane = (int)threadIdx.x;
-    JacD acc;
-    jacd_set_inf(acc);
-    if (lane < g.W) {
-        load_jacd(wins + kJacQ * ((uint64_t)s * g.W + lane), acc);
-        acc = jacd_dbl_n(acc, g.c * lane);
-    }
-    __syncwarp();
-    for (int d = 1; d < g.W; d <<= 1) {
-        const JacD o = shfl_jacd(acc, lane + d < 32 ? lane + d : lane);
-        if (lane + d < 32) acc = jacd_add(acc, o);
-    }
-    if (lane == 0) {
-        segok[s] = (uint8_t)((acc.inf ? 1 : 0) | (segbad[s] ? 2 : 0));
-        store_jacd(segpt + kJacQ * (uint64_t)s, acc);
-    }
-}
-
 inline unsigned grid_of(uint64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
 }  // namespace
 
-cudaError_t launch_rlc_windows(const RoundGeo& g, const uint4* buckets, uint4* wu, uint4* wt, uint4* wins,
-                               const uint32_t* segbad, uint8_t* segok, uint4* segpt, cudaStream_t s) {
+cudaError_t launch_rlc_windows(const RoundGeo& g, const uint4* buckets, uint4* wins, const uint32_t* segbad,
+                               uint8_t* segok, uint4* segpt, cudaStream_t s) {
     const uint64_t n_seg = g.n_seg;
-    k_rlc_wpart<<<grid_of(n_seg * g.W * g.S, 128), 128, 0, s>>>(g, buckets, wu, wt);
-    k_rlc_wcomb<<<grid_of(n_seg * g.W * g.S, 128), 128, 0, s>>>(g, wu, wt, wins);
-    if (g.W <= 32 && n_seg <= kWarpHornerSegments)
-        k_rlc_finish_warp<<<(unsigned)n_seg, 32, 0, s>>>(g, wins, segbad, segok, segpt);
-    else
-        k_rlc_finish<<<grid_of(n_seg, 32), 32, 0, s>>>(g, wins, segbad, segok, segpt);
+    const int threads = g.S > 32 ? g.S : 32;
+    k_rlc_window<<<grid_of(n_seg * g.W * g.S, threads), threads, 0, s>>>(g, buckets, wins);
+    int lanes = 32;                                // while the warps stay at one per scheduler
+    while (lanes > 1 && (n_seg * lanes > 592 * 32 || lanes >= 2 * g.W)) lanes >>= 1;
+    k_rlc_finish<<<grid_of(n_seg * lanes, 32), 32, 0, s>>>(g, lanes, wins, segbad, segok, segpt);
     return cudaGetLastError();
 }
 

@@ -14,7 +14,7 @@ namespace uf {
 // combination per window, and Horner over the windows per segment:
 // segok[s] = 1 when segment s's sum is infinity, | 2 when it holds an item
 // that failed to parse; segpt[s] = the sum.
-cudaError_t launch_rlc_windows(const rlcdev::RoundGeo& g, const uint4* buckets, uint4* wu, uint4* wt, uint4* wins,
+cudaError_t launch_rlc_windows(const rlcdev::RoundGeo& g, const uint4* buckets, uint4* wins,
                                const uint32_t* segbad, uint8_t* segok, uint4* segpt, cudaStream_t s);
 
 // Buckets of two or more chunks: the sum of their chunk partials, by a thread
