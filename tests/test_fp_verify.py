@@ -309,3 +309,20 @@ def test_jobs_packed_in_pieces(plain_ctx, oracle):
         want.append(ref[order])
     for got, ref in zip(plain_ctx.verify_jobs(jobs), want):
         assert (got == ref).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [4736, 4737, 9471, 9472])
+def test_two_warps_per_32_signatures(team_ctx, oracle, n):
+    """Around a block per SM (four warps up to it, two above) and two."""
+    check_sizes(team_ctx, oracle, n)
+
+
+@pytest.mark.gpu
+def test_two_warp_sums_that_meet(team_ctx, oracle):
+    em, ep, es, sm, sp, ss = meeting_signatures(oracle)
+    order = np.random.default_rng(3).integers(0, len(em), 4800)
+    assert (team_ctx.ecdsa_verify_batch(em[order], ep[order], es[order]) ==
+            oracle.ecdsa_verify_batch(em, ep, es)[order]).all()
+    order = np.random.default_rng(4).integers(0, len(sm), 4800)
+    assert not team_ctx.schnorr_verify_batch(sm[order], sp[order], ss[order]).any()

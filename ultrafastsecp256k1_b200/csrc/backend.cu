@@ -50,12 +50,12 @@ cudaError_t Backend::launch_verify(int kind, const uint8_t* m, const uint8_t* p,
                                    uint8_t* out, int collect, cudaStream_t st) {
     const int k = kind & 1;
     if (n <= pair_items_[k])
-        return launch_verify_team(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, st);
+        return launch_verify_team(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, sms_, st);
     const bool small = small_variant_[k] >= 0 && n <= small_items_[k];
     if (!small && inv_group_[k] > 1) {
         // A last wave of at most half a block per SM goes on its own, in smaller
         // blocks on every SM or in the small calls' form, instead of full blocks
-        // on some of them: 0.29 ms up to 32 items per SM, 0.44 up to 64 and 0.54
+        // on some of them: 0.29 ms up to 32 items per SM, 0.34 up to 64 and 0.54
         // up to 128 against 0.68 (50,021 signatures: 1.33 -> 1.21 ms).
         const uint32_t wave = (uint32_t)sms_ * 256u, tail = n % wave;
         if (n > wave && tail && tail <= wave / 2) {

@@ -85,20 +85,21 @@ int BatchSlot::init(Backend* be, bool use_graphs) {
     return kOk;
 }
 
-// Small launches run four warps per 32 signatures (the backend's tuned limit),
-// as long as what other slots have in flight leaves the device room for it: that
-// form halves a launch's time on an idle device (0.29 against 0.54 ms) and
-// halves the rate of a busy one (a burst of 96 requests, 47,000 signatures: 2.7
-// ms with it in every small launch, 2.3 with it up to the limit in flight).  The
-// choice is part of the graph key, so a graph captured with the other kernels is
-// never replayed.
-bool BatchSlot::small_launch(const QueueArgs& a) const {
+// Warps per 32 signatures of a small launch: four up to 32 items per SM, two up
+// to the backend's tuned limit (64 per SM), 0 (a thread each) above.  What other
+// slots have in flight counts too: sharing a signature halves a launch's time on
+// an idle device (0.29 against 0.54 ms) and costs rate on a busy one (a burst of
+// 96 requests, 47,000 signatures: 2.7 ms with four warps in every small launch,
+// 2.4 ms with them only up to the limits in flight).  The choice is part of the
+// graph key, so a graph captured with the other kernels is never replayed.
+int BatchSlot::team_warps(const QueueArgs& a) const {
     const uint64_t limit = be_->queue_pair_items();
-    return (uint64_t)a.cap_e + a.cap_s <= limit && beside_ <= limit;
+    const uint64_t items = std::max((uint64_t)a.cap_e + a.cap_s, beside_);
+    return items > limit ? 0 : (items > (uint64_t)be_->sms() * 32 ? 2 : 4);
 }
 
 uint64_t BatchSlot::graph_key(const QueueArgs& a) const {
-    return ((uint64_t)a.cap_e << 32) | a.cap_s | (small_launch(a) ? (1ull << 63) : 0);
+    return ((uint64_t)a.cap_e << 32) | a.cap_s | ((uint64_t)team_warps(a) << 61);
 }
 
 QueueArgs BatchSlot::args_for(uint8_t* d) const {
@@ -131,7 +132,7 @@ int BatchSlot::run_direct(const QueueArgs& a) {
     uint8_t* d = staged_big_ ? (uint8_t*)big_dev_.p : (uint8_t*)dev_.p;
     cudaError_t e = cudaMemcpyAsync(d, h, layout_.in_bytes, cudaMemcpyHostToDevice, stream_);
     if (e == cudaSuccess)
-        e = launch_verify_queue(a, small_launch(a), be_->gtab(), be_->comb(), be_->sms(),
+        e = launch_verify_queue(a, team_warps(a), be_->gtab(), be_->comb(), be_->sms(),
                                 QueueStreams{stream_, stream2_, stream3_, fork_, join_, join3_});
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h + layout_.e_out, d + layout_.e_out, layout_.out_bytes, cudaMemcpyDeviceToHost, stream_);
@@ -263,7 +264,7 @@ int BatchSlot::prewarm(uint32_t max_items) {
             hdr[1] = 0;
             hdr[2] = 0;
             const QueueArgs a = args_for((uint8_t*)dev_.p);
-            for (const uint64_t beside : {(uint64_t)0, ~(uint64_t)0}) {      // both forms of a small launch
+            for (const uint64_t beside : {(uint64_t)0, (uint64_t)be_->queue_pair_items(), ~(uint64_t)0}) {   // every form
                 beside_ = beside;
                 const int rc = run_graph(a, graph_key(a));
                 if (rc != kOk) return rc;

@@ -85,7 +85,7 @@ private:
 
     void pack(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, bool parallel);
     int run_direct(const QueueArgs& a);
-    bool small_launch(const QueueArgs& a) const;
+    int team_warps(const QueueArgs& a) const;
     uint64_t graph_key(const QueueArgs& a) const;
     int run_graph(const QueueArgs& a, uint64_t key);
     QueueArgs args_for(uint8_t* dev_base) const;

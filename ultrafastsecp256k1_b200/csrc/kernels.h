@@ -83,9 +83,10 @@ cudaError_t launch_verify_fp(int kind, const uint8_t* msgs, const uint8_t* pubs,
                              const void* d_gtab, const void* d_comb, uint8_t* out, int collect, int sms,
                              cudaStream_t s);
 cudaError_t verify_fp_init();
-// Small calls: four warps per 32 signatures (kernels_team.cu).
+// Small calls: four or two warps per 32 signatures (kernels_team.cu).
 cudaError_t launch_verify_team(int kind, const uint8_t* msgs, const uint8_t* pubs, const uint8_t* sigs, uint32_t n,
-                               const void* d_gtab, const void* d_comb, uint8_t* out, int collect, cudaStream_t s);
+                               const void* d_gtab, const void* d_comb, uint8_t* out, int collect, int sms,
+                               cudaStream_t s);
 cudaError_t verify_team_init();
 // Fills the generator window table (comb_table_bytes() bytes; isocheck.cuh).
 size_t comb_table_bytes();
@@ -161,11 +162,12 @@ struct QueueStreams {
 
 // Launches the verify kernels over the items described by `a` (kernels_queue.cu):
 // kinds with capacity 0 are skipped; with both kinds, the BIP-340 kernel runs on
-// its own branch.  team: four warps per 32 signatures (small launches).  With a
+// its own branch.  team_warps: four or two warps per 32 signatures (small
+// launches), or 0.  With a
 // key table (a.cache) the resolve and build passes (pubcache.cuh) run first, for
 // team launches beside the verify kernels.  verify_queue_init opts the kernels in
 // to their shared memory (once per device).
-cudaError_t launch_verify_queue(const QueueArgs& a, bool team, const void* d_gtab, const void* d_comb, int sms,
+cudaError_t launch_verify_queue(const QueueArgs& a, int team_warps, const void* d_gtab, const void* d_comb, int sms,
                                 const QueueStreams& q);
 cudaError_t verify_queue_init();
 

@@ -157,24 +157,25 @@ k_verify_queue(QueueArgs a, const uint4* __restrict__ gt, const uint4* __restric
     if (valid) (kKind == 0 ? a.e_out : a.s_out)[i] = ok ? 1 : 0;
 }
 
-template <int kKind>
-__global__ void __launch_bounds__(kTeamThreads, 2)
+template <int kKind, int kWarps>
+__global__ void __launch_bounds__(kWarps * kTeamLanes, 8 / kWarps)
 k_verify_queue_team(QueueArgs a, const uint4* __restrict__ gt, const uint4* __restrict__ comb) {
     extern __shared__ uint4 smem[];
     const uint32_t total = kKind == 0 ? min(a.counts[0], a.cap_e) : min(a.counts[1], a.cap_s);
     if (blockIdx.x * kTeamLanes >= total) return;          // the whole block
     const uint32_t i = blockIdx.x * kTeamLanes + (threadIdx.x & 31u);
-    const bool ok = team_verify<kKind>((kKind == 0 ? a.e_msgs : a.s_msgs) + 32ull * i,
+    const bool ok = team_verify<kKind, kWarps>((kKind == 0 ? a.e_msgs : a.s_msgs) + 32ull * i,
                                        kKind == 0 ? a.e_pubs + 33ull * i : a.s_pubs + 32ull * i,
                                        (kKind == 0 ? a.e_sigs : a.s_sigs) + 64ull * i, i < total, gt, comb, smem);
     if (threadIdx.x < kTeamLanes && i < total) (kKind == 0 ? a.e_out : a.s_out)[i] = ok ? 1 : 0;
 }
 
-cudaError_t launch_verify_queue(const QueueArgs& a, bool team, const void* d_gtab, const void* d_comb, int sms,
+cudaError_t launch_verify_queue(const QueueArgs& a, int team_warps, const void* d_gtab, const void* d_comb, int sms,
                                 const QueueStreams& q) {
     const uint4* gt = reinterpret_cast<const uint4*>(d_gtab);
     const uint4* comb = reinterpret_cast<const uint4*>(d_comb);
     cudaError_t e = cudaSuccess;
+    const bool team = team_warps != 0;
     const bool both = a.cap_e > 0 && a.cap_s > 0;
     if (!team && (e = launch_key_passes(a, sms, q.main)) != cudaSuccess) return e;
     const bool beside = team && a.cache;                   // the key passes on a branch of their own
@@ -186,8 +187,13 @@ cudaError_t launch_verify_queue(const QueueArgs& a, bool team, const void* d_gta
     cudaStream_t ss = both ? q.second : q.main;
     if (team) {
         const unsigned ge = (a.cap_e + kTeamLanes - 1) / kTeamLanes, gs = (a.cap_s + kTeamLanes - 1) / kTeamLanes;
-        if (ge) k_verify_queue_team<0><<<ge, kTeamThreads, kTeamSmem, q.main>>>(a, gt, comb);
-        if (gs) k_verify_queue_team<1><<<gs, kTeamThreads, kTeamSmem, ss>>>(a, gt, comb);
+        if (team_warps == 4) {
+            if (ge) k_verify_queue_team<0, 4><<<ge, kTeamThreads, kTeamSmem, q.main>>>(a, gt, comb);
+            if (gs) k_verify_queue_team<1, 4><<<gs, kTeamThreads, kTeamSmem, ss>>>(a, gt, comb);
+        } else {
+            if (ge) k_verify_queue_team<0, 2><<<ge, kDuoThreads, kTeamSmem, q.main>>>(a, gt, comb);
+            if (gs) k_verify_queue_team<1, 2><<<gs, kDuoThreads, kTeamSmem, ss>>>(a, gt, comb);
+        }
     } else {
         // full blocks, one per SM, for launches that fill the device; two half
         // blocks per SM where both kinds or a part of a wave share it
@@ -222,8 +228,10 @@ cudaError_t verify_queue_init() {
     opt_in(k_verify_queue<false, 1>, full);
     opt_in(k_verify_queue<true, 0>, full);
     opt_in(k_verify_queue<true, 1>, full);
-    opt_in(k_verify_queue_team<0>, kTeamSmem);
-    opt_in(k_verify_queue_team<1>, kTeamSmem);
+    opt_in(k_verify_queue_team<0, 4>, kTeamSmem);
+    opt_in(k_verify_queue_team<1, 4>, kTeamSmem);
+    opt_in(k_verify_queue_team<0, 2>, kTeamSmem);
+    opt_in(k_verify_queue_team<1, 2>, kTeamSmem);
     opt_in(k_key_build, kBuildThreads * kFpSmemPerThread);
     return e;
 }

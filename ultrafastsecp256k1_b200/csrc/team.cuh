@@ -1,4 +1,4 @@
-// Small calls: four warps per 32 signatures.
+// Small calls: four or two warps per 32 signatures.
 //
 // A call of a few thousand signatures fills a fraction of the device, so its
 // time is one signature's chain of dependent operations.  Here lane l of each of
@@ -19,7 +19,9 @@
 // can.  The warps run the same code at the same time wherever that can be had:
 // with the whole generator sum on warp 0 beside the others' digits a third of
 // the issue slots waited for instructions (digits 390 k cycles instead of 325 k).
-// Up to two blocks share an SM, so it pays up to 2 x 32 signatures per SM.
+// It pays up to 32 signatures per SM, a warp for each of its schedulers; up to 64
+// two warps share 32 signatures the same way (kWarps = 2: the scalars beside the
+// table, all of the generator's windows after them).
 // Verdicts as in kernels_verify_fp.cu.
 #pragma once
 #include "verify_fp.cuh"
@@ -29,9 +31,11 @@ namespace uf {
 
 constexpr int kTeamLanes = 32;
 constexpr int kTeamThreads = 4 * kTeamLanes;
+constexpr int kDuoThreads = 2 * kTeamLanes;
 // digits [low, high) of each warp: equal times at 6.8 k cycles per three
 // doublings and as many per addition
 static __device__ const uint8_t kTeamLow[5] = {0, 23, 35, 41, kEisDigits};
+static __device__ const uint8_t kDuoLow[3] = {0, 29, kEisDigits};
 
 // Shared memory of a block, in 16-byte columns of one lane each.
 constexpr int kTabCells = 5 * kEisTab;       // the table
@@ -86,7 +90,7 @@ __device__ __forceinline__ JacD get_part(const double2* c) {
 // One signature per lane, verified by the block's four warps together (every
 // thread calls it; `valid` false for lanes without one, whose pointers are not
 // read).  The verdict is meaningful on warp 0.
-template <int kKind>
+template <int kKind, int kWarps = 4>
 __device__ __forceinline__ bool team_verify(const uint8_t* msg, const uint8_t* pub, const uint8_t* sig, bool valid,
                                             const uint4* gt, const uint4* comb, uint4* smem) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -128,7 +132,7 @@ __device__ __forceinline__ bool team_verify(const uint8_t* msg, const uint8_t* p
             scal[0] = make_uint4(a.v[0], a.v[1], a.v[2], a.v[3]);
             scal[kTeamLanes] = make_uint4(a.v[4], a.v[5], a.v[6], a.v[7]);
         }
-    } else if (kKind == 1 && ok) {
+    } else if (kKind == 1 && kWarps == 4 && ok) {
         uint32_t sw[8];
         Sc s;
         load_words8(sw, sig + 32);
@@ -136,6 +140,7 @@ __device__ __forceinline__ bool team_verify(const uint8_t* msg, const uint8_t* p
         const int half = (warp - 2) * (kCombWindows / 2);
         put_part(gen_c + warp * kPartCells * kTeamLanes, comb_mul<true>(s, comb, half, half + kCombWindows / 2));
     }
+    constexpr bool kGenAfter = kKind != 1 || kWarps == 2;      // the generator's windows shared by all warps
     // a lane goes on when no warp refused its item
     __shared__ uint32_t good[2];
     const uint32_t mine = __ballot_sync(0xFFFFFFFFu, ok);
@@ -144,41 +149,48 @@ __device__ __forceinline__ bool team_verify(const uint8_t* msg, const uint8_t* p
     ok = ((good[0] & good[1]) >> lane) & 1u;
     if (ok) {
         UF_NOUNROLL
-        for (int k = warp; k < kEisTab - 1; k += 4) {
+        for (int k = warp; k < kEisTab - 1; k += kWarps) {
             Fd rho;
             get_fd(rho, rho_c + 3 * k * kTeamLanes);
             eis_scale(tab, k, rho);
         }
-        if (kKind != 1) {
+        if (kGenAfter) {
             const uint4 lo = scal[0], hi = scal[kTeamLanes];
             const Sc a = {{lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}};
-            const int first = warp * (kCombWindows / 4);
-            put_part(gen_c + warp * kPartCells * kTeamLanes, comb_mul<true>(a, comb, first, first + kCombWindows / 4));
+            const int first = warp * (kCombWindows / kWarps);
+            put_part(gen_c + warp * kPartCells * kTeamLanes,
+                     comb_mul<true>(a, comb, first, first + kCombWindows / kWarps));
         }
     }
     __syncthreads();
     JacD A;
     jacd_set_inf(A);
     if (ok) {
-        const int low = kTeamLow[warp], high = kTeamLow[warp + 1];
+        const uint8_t* ranges = kWarps == 4 ? kTeamLow : kDuoLow;
+        const int low = ranges[warp], high = ranges[warp + 1];
         UF_NOUNROLL
         for (int q = high - 1; q >= 0; --q)
             eis_add_digit<true>(A, q >= low ? (uint32_t)dig[q * kTeamLanes] : kEisZero, q == high - 1, tab);
         if (warp != 0) put_part(part_c + (warp - 1) * kPartCells * kTeamLanes, A);
     }
     __syncthreads();
-    // first step: warps 0 and 2 on the key's sums, 1 and 3 on the generator's
     const int c1 = kPartCells * kTeamLanes;
-    if (ok) {
+    if (kWarps == 4) {
+        // first step: warps 0 and 2 on the key's sums, 1 and 3 on the generator's
+        if (ok) {
+            if (warp == 0) A = jacd_add(A, get_part(part_c));
+            if (warp == 2) put_part(part_c + c1, jacd_add(A, get_part(part_c + 2 * c1)));
+            if (warp == 1 && kKind != 1) put_part(gen_c, jacd_add(get_part(gen_c), get_part(gen_c + c1)));
+            if (warp == 3) put_part(gen_c + 2 * c1, jacd_add(get_part(gen_c + 2 * c1), get_part(gen_c + 3 * c1)));
+        }
+        __syncthreads();
+        if (ok) {
+            if (warp == 0) A = jacd_add(A, get_part(part_c + c1));
+            if (warp == 1 && kKind != 1) put_part(gen_c + 2 * c1, jacd_add(get_part(gen_c), get_part(gen_c + 2 * c1)));
+        }
+    } else if (ok) {
         if (warp == 0) A = jacd_add(A, get_part(part_c));
-        if (warp == 2) put_part(part_c + c1, jacd_add(A, get_part(part_c + 2 * c1)));
-        if (warp == 1 && kKind != 1) put_part(gen_c, jacd_add(get_part(gen_c), get_part(gen_c + c1)));
-        if (warp == 3) put_part(gen_c + 2 * c1, jacd_add(get_part(gen_c + 2 * c1), get_part(gen_c + 3 * c1)));
-    }
-    __syncthreads();
-    if (ok) {
-        if (warp == 0) A = jacd_add(A, get_part(part_c + c1));
-        if (warp == 1 && kKind != 1) put_part(gen_c + 2 * c1, jacd_add(get_part(gen_c), get_part(gen_c + 2 * c1)));
+        if (warp == 1) put_part(gen_c + 2 * c1, jacd_add(get_part(gen_c), get_part(gen_c + c1)));
     }
     __syncthreads();
     if (warp != 0 || !ok) return false;
