@@ -15,9 +15,12 @@ by the tests).
   max over ranks.
 * e2e: the same work through the reference ABI call
   ufsecp_gpu_schnorr_verify_batch with host buffers, copies included.
-* roofline: integer-pipe (IMAD) bound; achieved = sigs/s x the canonical
-  3.33e5 IMAD-class ops per signature, against the device's IMAD issue rate
-  measured in this run; HBM bytes of the same launch beside it.
+* roofline: FP64 pipe; achieved = sigs/s x the 1.70e5 FP64 operations per
+  signature that the headline kernel issues (ncu, profiles/k_verify_fp_bip340.md),
+  against the pipe's rate (64 lanes per SM and cycle).  Three-register operations
+  take 3.1 cycles instead of 2 (register reads), so about 0.6 is the practical top.
+  `model`: the canonical 3.33e5 IMAD-class operations per signature against the IMAD
+  rate measured in this run; HBM bytes of the same launch beside it.
 * cpu_baseline: the reference library (oracle/_ref, compiled from the
   reference sources) on all host threads over a bounded sample.
 Multi-GPU: one process per GPU (torchrun), every rank verifies its own batch
@@ -44,6 +47,7 @@ METRIC = "verified sigs/sec on 1 B200 (ECDSA, BIP-340) batched vs plain kernel; 
 N_ORDER = 0xFFFFFFFFFFFFFFFFFFFFFFFFFFFFFFFEBAAEDCE6AF48A03BBFD25E8CD0364141
 P_FIELD = 2**256 - 2**32 - 977
 W_SIG = 3.33e5            # IMAD-class ops per verified signature (canonical work model)
+W_FP64 = 1.70e5           # FP64 operations per signature of the headline kernel
 BYTES_PER_SIG = 32 + 32 + 64 + 1
 BATCH = 1 << 20
 CPU_SAMPLE = 1 << 20            # the whole headline batch
@@ -201,10 +205,10 @@ def make_schnorr_batch(ctx, torch, n: int, seed: int, invalid: bool = True):
 
 
 def launches_per_call(n: int) -> int:
-    """Kernel launches of one ufsecp_gpu_ext_schnorr_verify_device call over n items
-    (large calls are cut into launches of 131,072 on two streams)."""
-    chunk = 1 << 17
-    return 1 if n < 2 * chunk else -(-n // chunk)
+    """Kernel launches of one ufsecp_gpu_ext_schnorr_verify_device call over n items on
+    148 SMs: one, and another for a last wave of at most 128 items per SM."""
+    wave = 148 * 256
+    return 2 if n > wave and 0 < n % wave <= wave // 2 else 1
 
 
 def cpu_reference_rate(msgs, xs, sigs, sample: int):
@@ -378,8 +382,10 @@ def run_ours(args):
         traffic = profile_traffic().get("k_verify_schnorr_bytes_per_sig")
         per_launch_s = avg_launch_ms * 1e-3
         sigs_per_rank_s = n / per_launch_s
-        achieved = sigs_per_rank_s * W_SIG / 1e9
-        peak = imad_peak / 1e9
+        model = sigs_per_rank_s * W_SIG / 1e9
+        achieved = sigs_per_rank_s * W_FP64 / 1e9
+        sm_mhz = (clocks or {}).get("sm_max_mhz") or 1965.0
+        peak = torch.cuda.get_device_properties(local).multi_processor_count * 64 * sm_mhz / 1e3
         hbm_peak = peaks.get("hbm_gbs", 6650.0)
         hbm_achieved = n * BYTES_PER_SIG / per_launch_s / 1e9
         line = {
@@ -395,11 +401,15 @@ def run_ours(args):
             "e2e": {"value": e2e_value, "unit": "sigs/s", "h2d_bytes_per_step": n * 128, "d2h_bytes_per_step": n,
                     "api": "ufsecp_gpu_schnorr_verify_batch (host buffers)",
                     "verdict_agreement": e2e_agree / n},
-            "roofline": {"bound": "int", "achieved": achieved, "peak": peak, "unit": "Gop/s",
+            "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "Gop/s",
                          "frac": achieved / peak if peak else None,
                          "traffic": (traffic * n) if traffic else None,
-                         "ops_per_sig": W_SIG, "launch_ms": avg_launch_ms,
-                         "peak_source": "measured in this run: 32-bit IMAD issue rate (ufsecp_gpu_ext_imad_peak)",
+                         "ops_per_sig": W_FP64, "launch_ms": avg_launch_ms,
+                         "peak_source": "64 FP64 lanes per SM x SMs x the maximum SM clock",
+                         "model": {"achieved": model, "peak": imad_peak / 1e9, "unit": "Gop/s",
+                                   "ops_per_sig": W_SIG,
+                                   "peak_source": "measured in this run: 32-bit IMAD issue rate "
+                                                  "(ufsecp_gpu_ext_imad_peak)"},
                          "hbm": {"achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
                                  "frac": hbm_achieved / hbm_peak, "peak_source": "of measured (MEASURED_PEAKS.json)"}},
             "cpu_baseline": cpu,

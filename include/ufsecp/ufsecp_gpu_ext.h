@@ -96,9 +96,8 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_inject_fault(ufsecp_gpu_ctx* ctx, uint3
 
 /* Resident key table of ufsecp_gpu_ext_verify_jobs (no reference
  * counterpart).  Per distinct public key (x, parity) a device slot keeps the
- * decompressed key's 1P..8P table, so a key seen before skips its square root,
- * table additions and the table's inversion; an x off the curve is remembered
- * as such.  Before the verify kernels, a resolve pass gives each item its key's
+ * decompressed key's table of 11 multiples, so a key seen before skips its
+ * table's additions; an x off the curve is remembered as such.  Before the verify kernels, a resolve pass gives each item its key's
  * slot and a build pass fills the new slots, so the verify warps never mix
  * lanes that build a table with lanes that copy one.  Verdicts never depend on
  * the table.  log2_slots: 0 = off; 8..24 = an empty table of 2^log2_slots
@@ -230,10 +229,10 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_schnorr_batch_identify_invalid(ufsecp_g
  * UFSECP_ERR_GPU_QUEUE on timeout (the request stays pending).  While a server
  * runs, its context belongs to the server's thread: make no other call on that
  * context.  Destroy the server (it finishes the pending requests) before the
- * context.  With key_cache_log2 set, decompressed keys with their 1P..8P
+ * context.  With key_cache_log2 set, decompressed keys with their
  * tables stay resident in a device key table shared by the slots (the design
- * of ufsecp_gpu_ext_set_key_table), so a key seen before skips its square
- * root, table additions and inversion (verdicts are unchanged).  The memory
+ * of ufsecp_gpu_ext_set_key_table), so a key seen before skips its
+ * table's additions (verdicts are unchanged).  The memory
  * budget covers the slots' fixed staging (pinned + device) and the key table,
  * reserved at creation (fewer slots are made if they do not fit), plus the
  * staged bytes of the items in flight; pending requests wait for room.
@@ -361,8 +360,8 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_set_small_variant(ufsecp_gpu_ctx* ctx, 
                                                            uint32_t items);
 
 /* Several threads per signature (kind 0 ECDSA, 1 BIP-340): with lanes = 2, calls
- * of at most `items` items cut each signature's work between threads (plain
- * calls between four warps of a block, mixed-job launches between two lanes): a
+ * of at most `items` items cut each signature's work between threads (four warps
+ * of a block work on 32 signatures, above 32 signatures per SM two warps): a
  * shorter verify latency for more arithmetic in all, which pays while the device
  * has idle capacity (small calls).  lanes = 1 turns it off.  The tuning file sets
  * it per kind (ecdsa_pair_items / schnorr_pair_items); set_variant turns it off.
@@ -376,7 +375,7 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_get_lanes(ufsecp_gpu_ctx* ctx, int kind
  * 128 = the kernel on the FP64 pipe that needs one inversion per BIP-340
  * signature and two per ECDSA one (both values mean the same kernel; they were
  * the thread counts of kernels that shared inversions inside a block).  Applies
- * to the main verify launches, not to the two-lane or small-launch paths.  The
+ * to the main verify launches, not to the lanes or small-launch paths.  The
  * tuning file sets it per kind (ecdsa_inv_group / schnorr_inv_group, chosen by
  * the autotuner); UFSECP_B200_INV_GROUP overrides both kinds; set_variant resets
  * the kind to 1.  Verdicts do not depend on it. */

@@ -7,10 +7,11 @@ For each signature kind (ECDSA, BIP-340) it times every verify-kernel variant
 arithmetic is inlined, i.e. instruction-cache footprint against call
 overhead, 9..11 in the P / G window widths: 3 / 18, 5 / 20, 4 / 16 bits
 against the default 4 / 20) on a GPU-signed batch, checks that all variants return identical
-verdicts, and picks them, plus the inversion group (threads of a block that
-share each modular inversion: 1, 64 or 128), a small-launch variant and its
-item limit for latency-bound launches (a few warps per SM) and the call size
-up to which two lanes per signature beat one; then, for RLC batch verification, it times the
+verdicts, and picks them, plus the main kernel ("inversion group" 1: that
+variant, 64 or 128: the FP64 kernel), where the variant stays the main kernel a
+small-launch variant and its item limit for latency-bound launches (a few warps
+per SM), and the launch size up to which four or two warps per 32 signatures beat
+a thread each; then, for RLC batch verification, it times the
 Pippenger window width (the MSM bucket width, 2^(c-1) buckets per window)
 for each batch size of 64 / 512 / 4096 / 16384 over the model's choice and
 its neighbours and picks the fastest.  The winners go to a tuning file of
@@ -83,7 +84,8 @@ def time_variant(ctx, torch, kind, bufs, n, reps=3):
     return n / (ms * 1e-3), out.cpu().numpy()
 
 
-SMALL_SIZES = (4096, 8192, 16384, 32768, 65536)
+# 32, 64, 128 and 256 items per SM of a 148-SM device, and above
+SMALL_SIZES = (4736, 9472, 18944, 37888, 65536)
 
 
 def tune_small(ctx, torch, kind, bufs, main: int, reps: int = 10) -> dict:
@@ -110,9 +112,9 @@ def tune_small(ctx, torch, kind, bufs, main: int, reps: int = 10) -> dict:
 
 
 def tune_lanes(ctx, torch, kind, bufs, reps: int = 10) -> dict:
-    """Two lanes per signature against one, with the tuned (small-launch)
-    variants in place: the limit is the largest SMALL_SIZES entry up to which
-    two lanes stay faster (0: never)."""
+    """Four or two warps per 32 signatures against a thread each, with the tuned
+    main kernel in place: the limit is the largest SMALL_SIZES entry up to which
+    sharing stays faster (0: never)."""
     rates = {1: {}, 2: {}}
     for lanes in (1, 2):
         ctx.set_lanes(kind, lanes, 1 << 30)
@@ -132,10 +134,9 @@ INV_GROUPS = (1, 64, 128)
 
 
 def tune_inversion_group(ctx, torch, kind, bufs, n, ref, reps: int = 3) -> dict:
-    """Threads per block that share each modular inversion (Montgomery's trick
-    across a block, ufsecp_gpu_ext_set_inversion_group): 1 (every signature
-    alone, the tuned variant), 64 or 128, timed at the main batch size with the
-    main variant in place; every group must reproduce the verdicts."""
+    """Main kernel (ufsecp_gpu_ext_set_inversion_group): 1 (the tuned integer
+    variant) or 64 / 128 (the FP64 kernel), timed at the main batch size; each
+    must reproduce the verdicts."""
     rates = {}
     for g in INV_GROUPS:
         ctx.set_inversion_group(kind, g)
@@ -186,7 +187,7 @@ def tune_rlc(ctx, torch, total: int = 1 << 18, reps: int = 2) -> dict:
     return res
 
 
-RLC_CHUNKS = (4, 6, 8, 12, 16, 24, 32)
+RLC_CHUNKS = (12, 24, 48, 96, 160, 256)
 
 
 def tune_rlc_chunk(ctx, torch, windows: dict, total: int = 1 << 18, reps: int = 2) -> dict:
@@ -239,9 +240,13 @@ def autotune(batch: int = 1 << 18, out_path: str | None = None, write: bool = Tr
                     raise RuntimeError(f"variant {v} disagrees with variant 0 on {label}")
                 rates[v] = rate
             best = max(rates, key=rates.get)
-            small = tune_small(ctx, torch, kind, bufs, best)
             ctx.set_variant(kind, best)
             group = tune_inversion_group(ctx, torch, kind, bufs, batch, ref)
+            # the FP64 kernel is the faster one at every size: no integer variant beside it
+            small = {"variant": None, "items": 0}
+            if group["best"] == 1:
+                small = tune_small(ctx, torch, kind, bufs, best)
+                ctx.set_variant(kind, best)
             if small["variant"] is not None:
                 ctx.set_small_variant(kind, small["variant"], small["items"])
             res["kinds"][label] = {"sigs_per_s": {str(k): r for k, r in rates.items()}, "best": best,

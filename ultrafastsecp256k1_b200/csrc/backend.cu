@@ -130,7 +130,7 @@ int Backend::set_small_variant(int kind, int v, uint32_t items) {
 // Per-device tuning: a file of "key value" lines (ecdsa_variant,
 // schnorr_variant, their small-launch counterparts ecdsa_small_variant /
 // ecdsa_small_items and schnorr_small_variant / schnorr_small_items, the
-// two-lane limits ecdsa_pair_items / schnorr_pair_items, and
+// small-call limits ecdsa_pair_items / schnorr_pair_items, and
 // rlc_window_<batch>) written by ultrafastsecp256k1_b200.autotune.  It is the
 // file named by UFSECP_B200_TUNING, else tuning/<device name>_<SMs>sm.txt
 // beside the library's lib/ directory.  UFSECP_B200_VARIANT_ECDSA / _SCHNORR

@@ -117,7 +117,7 @@ public:
     bool rlc_locate() const { return rlc_locate_; }
     void set_rlc_locate(bool on) { rlc_locate_ = on; }
     // Mixed-job launches of at most this many items (both kinds together) run
-    // four warps per 32 signatures: the smaller of the kinds' limits.
+    // four or two warps per 32 signatures: the smaller of the kinds' limits.
     uint32_t queue_pair_items() const { return std::min(pair_items_[0], pair_items_[1]); }
     // Per-item batch operations (ops.cpp): host buffers, synchronous.
     int xonly_validate(const uint8_t* keys32, size_t n, uint8_t* out);
@@ -137,12 +137,10 @@ public:
     uint32_t small_items(int kind) const { return small_items_[kind & 1]; }
     int set_variant(int kind, int v);
     int set_small_variant(int kind, int v, uint32_t items);   // v = -1: none
-    int set_lanes(int kind, int lanes, uint32_t items);       // lanes 2 for calls of <= items, 1: never
-    // Inversion group per kind: 1 = every signature inverts alone (the
-    // variant kernels), 64 / 128 = the block-wide batch-inversion kernels with
-    // that many threads per block share each inversion.  Applies to the main
-    // launches (not the two-lane or small-launch paths).  set_variant resets
-    // it to 1.
+    int set_lanes(int kind, int lanes, uint32_t items);       // 2: the small-call kernel for launches of <= items, 1: never
+    // Main kernel per kind: 1 = the integer variant kernels, 64 / 128 = the FP64
+    // kernel (kernels_verify_fp.cu).  Applies to the main launches (not the lanes
+    // or small-launch paths).  set_variant resets it to 1.
     int set_inversion_group(int kind, int group);
     int inversion_group(int kind) const { return inv_group_[kind & 1]; }
     uint32_t pair_items(int kind) const { return pair_items_[kind & 1]; }
@@ -183,7 +181,7 @@ private:
     int small_variant_[2] = {-1, -1};
     uint32_t small_items_[2] = {0, 0};
     // Launches of at most pair_items_[kind] items (kinds 0 and 1) run four
-    // warps per 32 signatures (kernels_team.cu); 0 = never.  Also cleared by an
+    // or two warps per 32 signatures (kernels_team.cu); 0 = never.  Also cleared by an
     // explicit variant choice.
     uint32_t pair_items_[2] = {0, 0};
     int inv_group_[2] = {1, 1};

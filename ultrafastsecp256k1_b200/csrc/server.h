@@ -13,7 +13,7 @@
 // Admission is bounded by a memory budget: the slots' fixed staging (pinned +
 // device, reserved at start) plus the staged bytes of the items of every launch
 // in flight stay within memory_budget_bytes.  Decompressed keys and their
-// 1P..8P tables stay resident in a device key table shared by all slots
+// tables stay resident in a device key table shared by all slots
 // (pubcache.cuh, keytable.h), so repeated keys skip decompression and table
 // set-up.  The verdicts of a request are the per-kind verify's, whatever it is
 // batched with.
