@@ -181,7 +181,7 @@ template <bool kCalls, class Tab>
 UF_HD void eis_add_digit(JacD& R, uint32_t e, bool top, const Tab& tab) {
     if (!top) {
         UF_NOUNROLL
-        for (int k = 0; k < 3; ++k) R = jacd_dbl_c(R);
+        for (int k = 0; k < 3; ++k) R = jacd_dbl_t<kCalls>(R);
     }
     if (e != kEisZero) {
         Fd x, y;
