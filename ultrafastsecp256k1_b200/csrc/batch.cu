@@ -163,13 +163,40 @@ int BatchSlot::run_graph(const QueueArgs& a, uint64_t key) {
     return kOk;
 }
 
-// The jobs' fields into the staging at h, in job order per kind: copies of at
-// most kPackBytes, handed out in runs of about that size.
+// fn(dst, src, bytes) for every field of the jobs, to the staging at h in job
+// order per kind.
+template <class F>
+void BatchSlot::each_field(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, F fn) {
+    size_t oe = 0, os = 0;
+    for (size_t j = 0; j < n_jobs; ++j) {
+        const VerifyJob& J = jobs[j];
+        if (J.count == 0) continue;
+        if (J.kind == 0) {
+            fn(h + layout_.e_msgs + 32 * oe, J.msgs, 32 * J.count);
+            fn(h + layout_.e_sigs + 64 * oe, J.sigs, 64 * J.count);
+            fn(h + layout_.e_pubs + 33 * oe, J.pubs, 33 * J.count);
+            oe += J.count;
+        } else {
+            fn(h + layout_.s_msgs + 32 * os, J.msgs, 32 * J.count);
+            fn(h + layout_.s_sigs + 64 * os, J.sigs, 64 * J.count);
+            fn(h + layout_.s_pubs + 32 * os, J.pubs, 32 * J.count);
+            os += J.count;
+        }
+    }
+}
+
+// The jobs' fields into the staging: by the calling thread, or in copies of at
+// most kPackBytes handed to the pool in runs of about that size.
 void BatchSlot::pack(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, bool parallel) {
+    if (!parallel) {
+        each_field(jobs, n_jobs, h, stage_copy);
+        stage_fence();
+        return;
+    }
     copies_.clear();
     runs_.assign(1, 0);
     size_t run = 0;
-    auto add = [&](uint8_t* dst, const uint8_t* src, size_t bytes) {
+    each_field(jobs, n_jobs, h, [&](uint8_t* dst, const uint8_t* src, size_t bytes) {
         while (bytes) {
             const size_t take = std::min(bytes, kPackBytes);
             copies_.push_back(Copy{dst, src, take});
@@ -182,34 +209,12 @@ void BatchSlot::pack(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, bool para
                 run = 0;
             }
         }
-    };
-    size_t oe = 0, os = 0;
-    for (size_t j = 0; j < n_jobs; ++j) {
-        const VerifyJob& J = jobs[j];
-        if (J.count == 0) continue;
-        if (J.kind == 0) {
-            add(h + layout_.e_msgs + 32 * oe, J.msgs, 32 * J.count);
-            add(h + layout_.e_sigs + 64 * oe, J.sigs, 64 * J.count);
-            add(h + layout_.e_pubs + 33 * oe, J.pubs, 33 * J.count);
-            oe += J.count;
-        } else {
-            add(h + layout_.s_msgs + 32 * os, J.msgs, 32 * J.count);
-            add(h + layout_.s_sigs + 64 * os, J.sigs, 64 * J.count);
-            add(h + layout_.s_pubs + 32 * os, J.pubs, 32 * J.count);
-            os += J.count;
-        }
-    }
+    });
     if (run) runs_.push_back((uint32_t)copies_.size());
-    auto one = [this](int p) {
+    be_->parallel_run((int)runs_.size() - 1, [this](int p) {
         for (uint32_t c = runs_[p]; c < runs_[p + 1]; ++c) stage_copy(copies_[c].dst, copies_[c].src, copies_[c].bytes);
         stage_fence();
-    };
-    const int parts = (int)runs_.size() - 1;
-    if (parallel) {
-        be_->parallel_run(parts, one);
-    } else {
-        for (int p = 0; p < parts; ++p) one(p);
-    }
+    });
 }
 
 int BatchSlot::enqueue(const VerifyJob* jobs, size_t n_jobs, size_t in_flight) {

@@ -83,6 +83,8 @@ private:
         size_t bytes;
     };
 
+    template <class F>
+    void each_field(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, F fn);
     void pack(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, bool parallel);
     int run_direct(const QueueArgs& a);
     int team_warps(const QueueArgs& a) const;
