@@ -414,7 +414,7 @@ UF_HD Fd fd_mul_sub_2sqr(Fd a, Fd b, Fd x) {
     return fd_reduce<FdBias<1, -2, 0, 1>, 1>(c);
 }
 
-UF_HD Fd fd_sqr_n(Fd a, int n) {
+UF_COLD Fd fd_sqr_n(Fd a, int n) {
     UF_NOUNROLL
     for (int i = 0; i < n; ++i) {
         uint64_t c[10];
@@ -468,6 +468,24 @@ UF_COLD Fd fdc_sub(Fd a, Fd b) {
     Fd r = fd_sub_l(a, b);
     fd_strict(r);
     return r;
+}
+
+// Whether a is a square mod p: its candidate root a^((p + 1) / 4), by the blocks of
+// ones of fe_sqrt_candidate (fe.cuh), squared.
+UF_COLD bool fd_is_square(Fd a) {
+    const Fd x2 = fdc_mul(fdc_sqr(a), a), x3 = fdc_mul(fdc_sqr(x2), a);
+    Fd t = fdc_mul(fd_sqr_n(x3, 3), x3);
+    t = fdc_mul(fd_sqr_n(t, 3), x3);
+    t = fdc_mul(fd_sqr_n(t, 2), x2);
+    const Fd x22 = fdc_mul(fd_sqr_n(t, 11), t), x44 = fdc_mul(fd_sqr_n(x22, 22), x22);
+    t = fdc_mul(fd_sqr_n(x44, 44), x44);
+    t = fdc_mul(fd_sqr_n(t, 88), t);
+    t = fdc_mul(fd_sqr_n(t, 44), x44);
+    t = fdc_mul(fd_sqr_n(t, 3), x3);
+    t = fdc_mul(fd_sqr_n(t, 23), x22);
+    t = fdc_mul(fd_sqr_n(t, 6), x2);
+    t = fd_sqr_n(t, 2);
+    return fd_is_zero(fdc_mul_sub(t, t, a));
 }
 
 }  // namespace uf

@@ -17,11 +17,26 @@
 // this y satisfies y^2 = c and has the parity; y^2 = c also shows that x is on
 // the curve (for a c that is no square no y passes).  BIP-340's y(R) follows as
 //   y_R = [(f c^2 za^3 - y b zb^3)(d - r zb^2) - f c za N] / (c za zb^3 N).
-// One inversion serves both.  It needs A, B finite and x_A != x_B: anything else
-// (only crafted signatures meet it) is left to the plain verification.
+// One inversion serves both.
+//
+// It needs A, B finite and x_A != x_B, and ECDSA's r may stand for r + n.  Only
+// crafted items meet these cases, but anyone can craft them, and one such item in
+// a block that verified it again alone held the block's SM for a second verify's
+// latency (1 % of them in 2^20 device-resident signatures: 47.4 - 49.4 ms against
+// 18.6).  So they take the same inversion, or none:
+//   x(R) = r + n: M is linear in r, so y(r + n) = (M - n cz zb^2 N^2) / g1.
+//   N = 0: y_A^2 = y_B^2 holds for either square root of c, so A = B or A = -B
+//     according to the parity of  y = f c^2 za^3 / (b zb^3);  then R = 2 B or
+//     infinity, and x(2 B), y(2 B) are compared (iso_meet; 1 % 19.1 ms).
+//   B infinite (ECDSA of a digest 0 mod n): x_A = r; that c is a square is looked at
+//     only where it holds (kIsoOnCurve; 1 % of such valid items 22.7 ms).
+//   A table whose Z is 0, or A infinite with b != 0: on secp256k1, whose order is a
+//     prime, neither happens (the table's path adds multiples of different small
+//     norm), so the key is not on it (1 % of points of small order 18.5 ms).
 #pragma once
 #include "common.cuh"
 #include "eis.cuh"
+#include "verify.cuh"
 
 namespace uf {
 
@@ -70,8 +85,10 @@ __device__ __forceinline__ JacD comb_mul(Sc s, const uint4* __restrict__ comb, i
     return B;
 }
 
+#endif  // __CUDACC__
+
 // The key on its scaled curve: (x c, c^2), c = x^3 + 7, from canonical limbs.
-__device__ __forceinline__ void iso_key(Fd& kx, Fd& ky, Fd& c, const uint32_t x[8]) {
+UF_HD void iso_key(Fd& kx, Fd& ky, Fd& c, const uint32_t x[8]) {
     Fd fx;
     fd_unpack(fx, x);
     fd_strict(fx);
@@ -93,20 +110,95 @@ __device__ __forceinline__ void iso_key(Fd& kx, Fd& ky, Fd& c, const uint32_t x[
 // resident key table) goes through the same check with c = 1: its scale is one,
 // so the equation holds exactly when y comes out as 1.
 //
-// iso_prepare returns false for A, B infinite or x_A = x_B; den = g1, for
-// BIP-340 g1 g2.
+// iso_prepare's den = g1, for BIP-340 g1 g2; slot 1 of an ECDSA item whose r may
+// stand for r + n holds what m loses for it.  Its result:
+enum : int {
+    kIsoNo = 0,        // the item is invalid
+    kIsoSolve = 1,     // iso_finish with 1 / den decides
+    kIsoOnCurve = 2,   // valid if the key is on the curve (iso_on_curve)
+    kIsoKeyInf = 3,    // BIP-340, b P infinite: b = 0, or the key is not on the curve
+    kIsoPlain = 4      // left to the plain verification (no item is known to get here)
+};
+
+// r + n as digits (r < p - n).
+UF_HD void iso_r_plus_n(Fd& f, const uint32_t r[8]) {
+    uint32_t w[8];
+    sc_n(w);
+    uint64_t t = 0;
+    UF_UNROLL
+    for (int i = 0; i < 8; ++i) {
+        t = (uint64_t)r[i] + w[i] + (t >> 32);
+        w[i] = lo32(t);
+    }
+    fd_unpack(f, w);
+    fd_strict(f);
+}
+
+// x(P) = r or, where alt, r + n, for a finite P (x = X / zz).
+UF_COLD bool iso_x_is(Fd X, Fd zz, Fd r, Fd rn, bool alt) {
+    if (fd_is_zero(fdc_mul_sub(r, zz, X))) return true;
+    return alt && fd_is_zero(fdc_mul_sub(rn, zz, X));
+}
+
+struct IsoDen {
+    Fd den;
+    int st;
+};
+
+// x_A = x_B.  y = u / v by the same slots and one more inverse, 1 / Z(2 B)^3, for
+// y(2 B): in iso_finish's terms m = u, g1 = v, g2 = Z^3, p1 = p2 = 0, p4 = -Y.
+// About 20 products more in a warp that holds such an item.
 template <bool kSchnorr, class Tab>
-__device__ __forceinline__ bool iso_prepare(const Tab& tab, Fd& den, const JacD& A, const JacD& B, const Fd& c,
-                                            const uint32_t r[8]) {
-    if (A.inf || B.inf) return false;
-    Fd fr;
+UF_COLD IsoDen iso_meet(Tab tab, JacD A, JacD B, Fd c, Fd r, Fd rn, bool alt) {
+    IsoDen o;
+    o.st = kIsoNo;
+    const JacD D = jacd_dbl_n(B, 1);
+    const Fd z2 = fdc_sqr(D.Z);
+    if (!iso_x_is(D.X, z2, r, rn, alt)) return o;
+    const Fd za3 = fdc_mul(fdc_sqr(A.Z), A.Z), zb3 = fdc_mul(fdc_sqr(B.Z), B.Z);
+    const Fd u = fdc_mul(fdc_mul(B.Y, c), fdc_mul(c, za3)), v = fdc_mul(A.Y, zb3);
+    Fd zero;
+    fd_set_u32(zero, 0);
+    o.st = kIsoSolve;
+    o.den = v;
+    tab.store(0, u, v);
+    if (kSchnorr) {
+        const Fd z3 = fdc_mul(z2, D.Z);
+        tab.store(1, zero, z3);
+        tab.store(2, zero, zero);
+        tab.store(3, fd_neg(D.Y), c);
+        o.den = fdc_mul(v, z3);
+    } else {
+        tab.store(1, zero, zero);
+        tab.store(3, c, c);
+    }
+    return o;
+}
+
+template <bool kSchnorr, class Tab>
+UF_HD int iso_prepare(const Tab& tab, Fd& den, const JacD& A, const JacD& B, const Fd& c, const uint32_t r[8]) {
+    if (A.inf) return kSchnorr ? kIsoKeyInf : kIsoNo;
+    Fd fr, frn;
     fd_unpack(fr, r);
     fd_strict(fr);
-    const Fd za2 = fdc_sqr(A.Z), zb2 = fdc_sqr(B.Z);
+    const bool alt = !kSchnorr && r_below_p_minus_n(r);
+    if (alt) iso_r_plus_n(frn, r);
+    else frn = fr;
+    const Fd za2 = fdc_sqr(A.Z);
     const Fd cz = fdc_mul(c, za2);
+    if (B.inf) {
+        if (kSchnorr) return kIsoPlain;
+        tab.store(3, c, c);
+        return iso_x_is(A.X, cz, fr, frn, alt) ? kIsoOnCurve : kIsoNo;
+    }
+    const Fd zb2 = fdc_sqr(B.Z);
     const Fd p2 = fdc_mul(A.X, zb2);
     const Fd N = fdc_mul_sub(B.X, cz, p2);
-    if (fd_is_zero(N)) return false;
+    if (fd_is_zero(N)) {
+        const IsoDen o = iso_meet<kSchnorr>(tab, A, B, c, fr, frn, alt);
+        den = o.den;
+        return o.st;
+    }
     const Fd za3 = fdc_mul(za2, A.Z), zb3 = fdc_mul(zb2, B.Z);
     const Fd c1 = fdc_mul(c, za3);
     const Fd g1 = fdc_mul(fdc_mul(fd_add_l(B.Y, B.Y), A.Y), fdc_mul(c1, zb3));
@@ -122,29 +214,45 @@ __device__ __forceinline__ bool iso_prepare(const Tab& tab, Fd& den, const JacD&
         tab.store(3, c, c);
     }
     // r cz zb^2 + a zb^2 + d cz, the last two as N + 2 a zb^2
-    const Fd K = fdc_add(fdc_add(fdc_mul(fr, fdc_mul(cz, zb2)), N), fd_add_l(p2, p2));
+    const Fd czb = fdc_mul(cz, zb2), N2 = fdc_sqr(N);
+    const Fd K = fdc_add(fdc_add(fdc_mul(fr, czb), N), fd_add_l(p2, p2));
     Fd m = fdc_mul(fdc_sqr(B.Y), fdc_mul(fdc_sqr(cz), cz));
     m = fdc_add(m, fdc_mul(fdc_sqr(A.Y), fdc_mul(fdc_sqr(zb2), zb2)));
-    m = fdc_sub(m, fdc_mul(K, fdc_sqr(N)));
+    m = fdc_sub(m, fdc_mul(K, N2));
     tab.store(0, m, g1);
-    return true;
+    if (alt) tab.store(1, fdc_mul(fdc_mul(czb, N2), fd_sub_l(frn, fr)), c);
+    return kIsoSolve;
+}
+
+template <class Tab>
+UF_HD bool iso_on_curve(const Tab& tab) {
+    Fd c, x;
+    tab.load(3, c, x);
+    return fd_is_square(c);
 }
 
 // Second half, with inv = 1 / den (canonical limbs).  unit: the key was given on
-// secp256k1 (c = 1).
+// secp256k1 (c = 1); alt: r < p - n (ECDSA).
 template <bool kSchnorr, class Tab>
-__device__ __forceinline__ bool iso_finish(const Tab& tab, const Fe& inv, bool odd, bool unit = false) {
+UF_HD bool iso_finish(const Tab& tab, const Fe& inv, bool odd, bool unit, bool alt) {
     Fd fi, m, g1, p1, g2, p4, c;
     fd_unpack(fi, inv.v);
     fd_strict(fi);
     tab.load(0, m, g1);
     tab.load(1, p1, g2);
     tab.load(3, p4, c);
-    const Fd y = fdc_mul(m, kSchnorr ? fdc_mul(fi, g2) : fi);
-    if (!fd_is_zero(fdc_mul_sub(y, y, c))) return false;
     uint32_t w[8];
+    Fd y = fdc_mul(m, kSchnorr ? fdc_mul(fi, g2) : fi);
+    bool good = fd_is_zero(fdc_mul_sub(y, y, c));
     fd_pack(w, y);
-    if (((w[0] & 1u) != 0) != (odd || unit)) return false;       // of +-1, 1 is the odd one
+    good = good && ((w[0] & 1u) != 0) == (odd || unit);          // of +-1, 1 is the odd one
+    if (!kSchnorr && !good && alt) {
+        y = fdc_mul(fdc_sub(m, p1), fi);
+        good = fd_is_zero(fdc_mul_sub(y, y, c));
+        fd_pack(w, y);
+        good = good && ((w[0] & 1u) != 0) == (odd || unit);
+    }
+    if (!good) return false;
     if (kSchnorr) {
         Fd p2, p3;
         tab.load(2, p2, p3);
@@ -155,7 +263,5 @@ __device__ __forceinline__ bool iso_finish(const Tab& tab, const Fe& inv, bool o
     }
     return true;
 }
-
-#endif  // __CUDACC__
 
 }  // namespace uf

@@ -5,9 +5,9 @@
 // unknown y, so that no square root is taken (isocheck.cuh), the generator's
 // multiple summed from a table of all windows, the field arithmetic in doubles
 // (fd.cuh).  The verdicts are those of ecdsa_verify_one / ecdsa_verify_opaque_one
-// / schnorr_verify_one (verify.cuh); what the scaled form does not cover (a sum
-// or an operand at infinity, equal x coordinates, an ECDSA r that may stand for
-// r + n) takes those functions themselves.
+// / schnorr_verify_one (verify.cuh); sums that meet or vanish and an ECDSA r that
+// may stand for r + n are decided in the scaled form too (isocheck.cuh), and those
+// functions themselves take only a BIP-340 challenge of 0.
 //
 // One block of 256 threads per SM, one item per thread: a thread's table is 11
 // points of ten doubles, 880 bytes of shared memory, read without conversion.

@@ -116,6 +116,7 @@ __device__ __forceinline__ bool team_verify(const uint8_t* msg, const uint8_t* p
                 put_fd(rho_c + 3 * k * kTeamLanes, zc);
                 if (k > 0) zc = fdc_mul(zc, hs[k]);
             }
+            ok = !fd_is_zero(zc);        // 0: the key is not on the curve (isocheck.cuh)
         }
     } else if (warp == 1) {
         uint32_t r[8];
@@ -202,21 +203,26 @@ __device__ __forceinline__ bool team_verify(const uint8_t* msg, const uint8_t* p
         fp_parse_sig<kKind>(r, s, sig);
     }
     Fd den;
-    bool plain = !iso_prepare<kKind == 1>(tab, den, A, B, c, r);
-    if (!plain) {
+    int st = iso_prepare<kKind == 1>(tab, den, A, B, c, r);
+    if (kKind == 1 && st == kIsoKeyInf) {
+        st = kIsoPlain;                         // e = 0, unless the key is not on the curve
+        for (int q = 0; q < kEisDigits; ++q)
+            if (dig[q * kTeamLanes] != kEisZero) st = kIsoNo;
+    }
+    bool holds = false;
+    if (st == kIsoSolve) {
         Fe inv;
         fd_pack(inv.v, den);
         if (is_zero256(inv.v)) {
-            plain = true;
+            st = kIsoPlain;
         } else {
             fe_inv(inv, inv);
-            ok = iso_finish<kKind == 1>(tab, inv, odd);
-            // x(R) may be r + n: the plain check looks at both
-            if (kKind != 1 && !ok && r_below_p_minus_n(r)) ok = plain = true;
+            holds = iso_finish<kKind == 1>(tab, inv, odd, false, kKind != 1 && r_below_p_minus_n(r));
         }
     }
-    if (plain) ok = plain_verify<kKind>(msg, pub, sig, gt, smem + lane, kTeamLanes);
-    return ok;
+    if (kKind != 1 && st == kIsoOnCurve) holds = iso_on_curve(tab);
+    if (st == kIsoPlain) holds = plain_verify<kKind>(msg, pub, sig, gt, smem + lane, kTeamLanes);
+    return holds;
 }
 
 }  // namespace uf

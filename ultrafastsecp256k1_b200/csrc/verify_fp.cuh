@@ -149,12 +149,12 @@ __device__ __forceinline__ bool fp_verify(const uint8_t* msg, const uint8_t* pub
     }
     Fd c, den, zc;
     JacD A;
-    bool plain = false;      // left to the plain verification
+    int st = kIsoNo;
     bool unit = false;       // the key's table comes from its slot
     if (kCached && ok && slot) {
-        const uint32_t st = slot_state(*slot);
-        unit = st == kSlotReady;
-        if (st == kSlotBad) ok = false;
+        const uint32_t state = slot_state(*slot);
+        unit = state == kSlotReady;
+        if (state == kSlotBad) ok = false;
     }
     __syncthreads();
     if (ok) {
@@ -179,6 +179,7 @@ __device__ __forceinline__ bool fp_verify(const uint8_t* msg, const uint8_t* pub
             Fd kx, ky;
             iso_key(kx, ky, c, px);
             zc = eis_table(tab, kx, ky);
+            ok = !fd_is_zero(zc);        // 0: the key is not on the curve (isocheck.cuh)
         }
     }
     jacd_set_inf(A);
@@ -202,23 +203,28 @@ __device__ __forceinline__ bool fp_verify(const uint8_t* msg, const uint8_t* pub
             load_words8(sw, sig);
             words_be_to_limbs(r, sw);
         }
-        plain = !iso_prepare<kKind == 1>(tab, den, A, B, c, r);
+        st = iso_prepare<kKind == 1>(tab, den, A, B, c, r);
+        if (kKind == 1 && st == kIsoKeyInf) {
+            st = kIsoPlain;                     // e = 0, unless the key is not on the curve
+            for (int q = 0; q < kEisDigits; ++q)
+                if (dig[q] != kEisZero) st = kIsoNo;
+        }
     }
     __syncthreads();
-    if (ok && !plain) {
+    bool holds = false;
+    if (st == kIsoSolve) {
         Fe inv;
         fd_pack(inv.v, den);
         if (is_zero256(inv.v)) {
-            plain = true;
+            st = kIsoPlain;
         } else {
             fe_inv(inv, inv);
-            ok = iso_finish<kKind == 1>(tab, inv, odd, unit);
-            // x(R) may be r + n: the plain check looks at both
-            if (kKind != 1 && !ok && r_below_p_minus_n(r)) ok = plain = true;
+            holds = iso_finish<kKind == 1>(tab, inv, odd, unit, kKind != 1 && r_below_p_minus_n(r));
         }
     }
-    if (ok && plain) ok = plain_verify<kKind>(msg, pub, sig, gt, smem + threadIdx.x, blockDim.x);
-    return ok;
+    if (kKind != 1 && st == kIsoOnCurve) holds = iso_on_curve(tab);
+    if (st == kIsoPlain) holds = plain_verify<kKind>(msg, pub, sig, gt, smem + threadIdx.x, blockDim.x);
+    return holds;
 }
 
 }  // namespace uf
