@@ -17,6 +17,7 @@
 #include "kernels.h"
 #include "pack_pool.h"
 #include "stage_copy.h"
+#include "host_chunks.h"
 #include "rlc.h"
 #include "nvtx.h"
 
@@ -47,11 +48,11 @@ int env_int(const char* name, int dflt) {
 }  // namespace
 
 cudaError_t Backend::launch_verify(int kind, const uint8_t* m, const uint8_t* p, const uint8_t* s, uint32_t n,
-                                   uint8_t* out, int collect, cudaStream_t st) {
+                                   uint8_t* out, int collect, cudaStream_t st, size_t call_items) {
     const int k = kind & 1;
     if (n <= pair_items_[k])
         return launch_verify_team(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, sms_, st);
-    const bool small = small_variant_[k] >= 0 && n <= small_items_[k];
+    const bool small = small_variant_[k] >= 0 && call_items <= small_items_[k];
     if (!small && inv_group_[k] > 1) {
         // A last wave of at most half a block per SM goes on its own, in smaller
         // blocks on every SM or in the small calls' form, instead of full blocks
@@ -63,7 +64,7 @@ cudaError_t Backend::launch_verify(int kind, const uint8_t* m, const uint8_t* p,
             const cudaError_t e = launch_verify_fp(kind, m, p, s, head, d_gtab_, d_comb_, out, collect, sms_, st);
             if (e != cudaSuccess) return e;
             return launch_verify(kind, m + 32ull * head, p + (kind == 1 ? 32ull : 33ull) * head, s + 64ull * head, tail,
-                                 out + head, collect, st);
+                                 out + head, collect, st, call_items);
         }
         return launch_verify_fp(kind, m, p, s, n, d_gtab_, d_comb_, out, collect, sms_, st);
     }
@@ -407,7 +408,7 @@ int Backend::verify_device(int kind, const uint8_t* d_msgs, const uint8_t* d_pub
     if (count < 2 * kDeviceChunk || inv_group_[kind & 1] > 1) {
         if (count >= 2 * kDeviceChunk)
             if (const int rc = fault_point("verify launch")) return rc;
-        e = launch_verify(kind, d_msgs, d_pubs, d_sigs, (uint32_t)count, d_out, 0, s);
+        e = launch_verify(kind, d_msgs, d_pubs, d_sigs, (uint32_t)count, d_out, 0, s, count);
         if (e != cudaSuccess) return cuda_error(e, "verify launch");
         clear_error();
         return kOk;
@@ -430,7 +431,7 @@ int Backend::verify_device(int kind, const uint8_t* d_msgs, const uint8_t* d_pub
     for (size_t off = 0; off < count; off += kDeviceChunk, ++k) {
         const size_t m = std::min(kDeviceChunk, count - off);
         e = launch_verify(kind, d_msgs + 32 * off, d_pubs + pub_sz * off, d_sigs + 64 * off, (uint32_t)m, d_out + off,
-                          0, (k & 1) ? dstream_ : s);
+                          0, (k & 1) ? dstream_ : s, count);
         if (e != cudaSuccess) return cuda_error(e, "verify launch");
     }
     if ((e = cudaEventRecord(djoin_, dstream_)) != cudaSuccess || (e = cudaStreamWaitEvent(s, djoin_, 0)) != cudaSuccess)
@@ -459,19 +460,16 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         }
         if (e != cudaSuccess) return cuda_error(e, "pipeline streams");
     }
-    // A chunk is one wave of the verify kernel (256 items per SM, 37,888 on a
-    // 148-SM B200): a smaller one would take the device as long as a full one
-    // once it holds more than 128 items per SM (0.68 ms; 0.54 below), and the
-    // CPU packs and copies in a wave in 0.2 ms.  Chunks rotate through
-    // kPipeSlots pinned staging slots: the CPU packs chunk k + 2 (and unpacks
-    // chunk k - 1's verdicts) while the device copies in and verifies chunks k
-    // and k + 1.  Per chunk the slot is laid out msgs | keys | sigs (16-byte
-    // aligned) | verdicts.
+    // Chunks (host_chunks.h) rotate through kPipeSlots pinned staging slots: the
+    // CPU packs chunk k + 2 (and unpacks chunk k - 1's verdicts) while the device
+    // copies in and verifies chunks k and k + 1.  Per chunk the slot is laid out
+    // msgs | keys | sigs (16-byte aligned) | verdicts.
     const size_t pub_sz = kind == 1 ? 32 : 33;
-    const size_t sub = std::min(count, (size_t)sms_ * 256);
+    const HostChunks chunks(inv_group_[kind & 1] > 1 ? (size_t)sms_ * 256 : 0);
+    const size_t sub = std::min(count, chunks.most);
     auto a16 = [](size_t v) { return (v + 15) & ~size_t{15}; };
     const size_t slot_bytes = a16(sub * (32 + pub_sz)) + sub * 64 + sub + 16;
-    const int slots = (int)std::min<size_t>(kPipeSlots, (count + sub - 1) / sub);
+    const int slots = (int)chunks.count(count, kPipeSlots);
     for (int j = 0; j < slots; ++j) {
         if ((e = pstage_[j].ensure(slot_bytes)) != cudaSuccess) return cuda_error(e, "cudaHostAlloc(staging)");
         if ((e = dstage_[j].ensure(slot_bytes)) != cudaSuccess) return cuda_error(e, "cudaMalloc(staging)");
@@ -497,7 +495,7 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         const int j = (int)(k % kPipeSlots);
         if ((e = drain(j)) != cudaSuccess) return fail(cuda_error(e, "verify"));
         if (const int rc = fault_point("verify launch")) return fail(rc);
-        m = std::min(sub, count - off);
+        m = chunks.size(k, count - off);
         const size_t o_p = m * 32, o_s = a16(o_p + m * pub_sz), o_o = o_s + m * 64;
         uint8_t* h = (uint8_t*)pstage_[j].p;
         uint8_t* d = (uint8_t*)dstage_[j].p;
@@ -528,12 +526,10 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         if ((e = field(0, msgs, 32, m_stride)) != cudaSuccess || (e = field(o_p, pubs, pub_sz, p_stride)) != cudaSuccess ||
             (e = field(o_s, sigs, 64, s_stride)) != cudaSuccess)
             return fail(cuda_error(e, "host->device copy"));
-        // a last chunk of at most half a wave waits for the one before it: its
-        // small blocks would fill the first SMs to finish, two by two
-        if (k > 0 && m <= sub / 2 &&
+        if (chunks.after_previous(k, m) &&
             (e = cudaStreamWaitEvent(pstream_[j], pev_[(k - 1) % kPipeSlots], 0)) != cudaSuccess)
             return fail(cuda_error(e, "event wait"));
-        e = launch_verify(kind, d, d + o_p, d + o_s, (uint32_t)m, d + o_o, collect, pstream_[j]);
+        e = launch_verify(kind, d, d + o_p, d + o_s, (uint32_t)m, d + o_o, collect, pstream_[j], count);
         if (e != cudaSuccess) return fail(cuda_error(e, "verify launch"));
         if ((e = cudaMemcpyAsync(h + o_o, d + o_o, m, cudaMemcpyDeviceToHost, pstream_[j])) != cudaSuccess)
             return fail(cuda_error(e, "device->host copy"));

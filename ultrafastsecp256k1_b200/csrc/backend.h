@@ -185,8 +185,11 @@ private:
     // explicit variant choice.
     uint32_t pair_items_[2] = {0, 0};
     int inv_group_[2] = {1, 1};
+    // call_items: the size of the whole call this launch belongs to, which the
+    // small-launch variant goes by (the chunks of a large call run beside one
+    // another); the small-call form goes by the launch.
     cudaError_t launch_verify(int kind, const uint8_t* m, const uint8_t* p, const uint8_t* s, uint32_t n,
-                              uint8_t* out, int collect, cudaStream_t st);
+                              uint8_t* out, int collect, cudaStream_t st, size_t call_items);
     void load_tuning();
     cudaStream_t stream_ = nullptr;
     void* d_gtab_ = nullptr;
