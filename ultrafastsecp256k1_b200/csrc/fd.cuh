@@ -20,11 +20,17 @@
 // constant plus q and a constant plus the low half: they are summed per column
 // as integers and the constants leave with the column's initial value.
 //
-// Digits.  "Strict" digits d_0..d_3 lie in [-2^51, 2^51] and |d_4| < 2^48; every
-// function below returns strict digits unless it says otherwise, and the value
-// of a multiplication's result is in (-p, p).  A product may take strict digits
-// times sums or differences of two strict values (2^52 * 2^51 = 2^103), or
-// times the unsigned digits [0, 2^52) of an unpacked table coordinate.
+// Digits.  "Strict" digits d_0..d_3 lie in [-2^51, 2^51]; every function below
+// returns strict digits unless it says otherwise, and a multiplication's result
+// has |d_4| <= 2^47 + 2^12 and its value in (-p, p), which fd_pack and fd_is_zero
+// need.  A product may take strict digits times sums or differences of two strict
+// values (2^52 * 2^51 = 2^103), or times the unsigned digits [0, 2^52) of an
+// unpacked table coordinate.
+//
+// The top digit of other values is larger: 2^48 for a coordinate just below p,
+// 2^49 for sums of a few results.  Products take |d_4| up to 2^50: the column of
+// weight 2^468 holds the top products' high halves alone, so those of one
+// reduction have to stay below 2^103 together (a b - 2 x^2: 3 * 2^100).
 #pragma once
 #include "common.cuh"
 #include "fe.cuh"
@@ -299,8 +305,8 @@ UF_HD void fd_unpack(Fd& r, const uint32_t w[8]) {
     r.v[4] = fd_mk((w[7] >> 16) | UF_FD_EXP, (w[6] >> 16) | (w[7] << 16)) - UF_FD_2P52;
 }
 
-// Any digits below 2^53 in magnitude with |v_4| <= 2^48 - 2 -> strict digits of
-// the same value.
+// Any digits below 2^53 in magnitude -> strict digits of the same value (what the
+// lower digits carry goes to the top one).
 UF_HD void fd_strict(Fd& a) {
     UF_UNROLL
     for (int k = 0; k < 4; ++k) {
@@ -457,6 +463,7 @@ UF_COLD Fd fdc_mul(Fd a, Fd b) { return fd_mul(a, b); }
 UF_COLD Fd fdc_sqr(Fd a) { return fd_sqr(a); }
 UF_COLD Fd fdc_mul_sub(Fd a, Fd b, Fd x) { return fd_mul_sub(a, b, x); }
 UF_COLD Fd fdc_sqr_sub_sub(Fd a, Fd x, Fd y) { return fd_sqr_sub_sub(a, x, y); }
+UF_COLD Fd fdc_sqr_sub_sub2(Fd a, Fd x, Fd y) { return fd_sqr_sub_sub2(a, x, y); }
 
 // a + b and a - b as strict digits
 UF_COLD Fd fdc_add(Fd a, Fd b) {

@@ -244,6 +244,7 @@ UF_HD bool iso_finish(const Tab& tab, const Fe& inv, bool odd, bool unit, bool a
     uint32_t w[8];
     Fd y = fdc_mul(m, kSchnorr ? fdc_mul(fi, g2) : fi);
     bool good = fd_is_zero(fdc_mul_sub(y, y, c));
+    if (kSchnorr && !good) return false;
     fd_pack(w, y);
     good = good && ((w[0] & 1u) != 0) == (odd || unit);          // of +-1, 1 is the odd one
     if (!kSchnorr && !good && alt) {

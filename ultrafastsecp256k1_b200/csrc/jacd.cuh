@@ -197,7 +197,7 @@ UF_COLD JacD jacd_add(JacD a, JacD b) {
     const Fd HH = fdc_sqr(H);
     const Fd HHH = fdc_mul(H, HH), V = fdc_mul(U, HH);
     a.Z = fdc_mul(fdc_mul(a.Z, b.Z), H);
-    a.X = fdc_sub(fdc_sqr_sub_sub(r, HHH, V), V);
+    a.X = fdc_sqr_sub_sub2(r, HHH, V);         // one reduction: a difference of two may leave (-p, p)
     a.Y = fdc_mul_sub(fd_sub_l(V, a.X), r, fdc_mul(S, HHH));
     return a;
 }
