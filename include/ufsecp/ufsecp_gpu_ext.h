@@ -234,7 +234,8 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_schnorr_batch_identify_invalid(ufsecp_g
  * of ufsecp_gpu_ext_set_key_table), so a key seen before skips its
  * table's additions (verdicts are unchanged).  The memory
  * budget covers the slots' fixed staging (pinned + device) and the key table,
- * reserved at creation (fewer slots are made if they do not fit), plus the
+ * reserved at creation (fewer slots are made if they do not fit; a key table
+ * that fits only to three quarters beside one slot is made half as large), plus the
  * staged bytes of the items in flight; pending requests wait for room.
  * Config NULL = defaults: 8 slots, 65,536 items per launch, an 8 GiB budget,
  * no batch window, a key table of 2^18 slots. */

@@ -1,6 +1,7 @@
 // Serving loop implementation (see server.h).
 #include "server.h"
 #include "nvtx.h"
+#include "server_budget.h"
 
 #include <cuda_runtime.h>
 
@@ -34,10 +35,11 @@ int Server::start(const ServerConfig& cfg) {
     if (cfg_.key_cache_log2 != 0 &&
         (cfg_.key_cache_log2 < KeyTable::kMinLog2 || cfg_.key_cache_log2 > KeyTable::kMaxLog2))
         return be_->set_error(kErrBadInput, "key_cache_log2 must be 0 or 8..24");
-    const uint64_t cache_bytes =
-        cfg_.key_cache_log2 ? (kPubCacheSlotBytes << cfg_.key_cache_log2) + 256 : 0;
-    if (cfg_.memory_budget_bytes < slot_bytes + cache_bytes)
-        return be_->set_error(kErrBadInput, "memory budget below one slot and the key cache");
+    const int fit = key_table_fit(cfg_.key_cache_log2, KeyTable::kMinLog2, kPubCacheSlotBytes,
+                                  cfg_.memory_budget_bytes, slot_bytes);
+    if (fit < 0) return be_->set_error(kErrBadInput, "memory budget below one slot and the key cache");
+    cfg_.key_cache_log2 = (uint32_t)fit;
+    const uint64_t cache_bytes = key_table_bytes(cfg_.key_cache_log2, kPubCacheSlotBytes);
     cfg_.slots = (uint32_t)std::min<uint64_t>(
         cfg_.slots, std::max<uint64_t>(1, (cfg_.memory_budget_bytes - cache_bytes) / slot_bytes));
     if (cfg_.key_cache_log2) {
