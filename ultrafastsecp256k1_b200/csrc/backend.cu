@@ -482,19 +482,24 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         pend_n[j] = 0;
         return r;
     };
-    // every early return waits for the slots' streams first, so that no copy
-    // of this call is still in flight when the next call packs a slot
-    auto fail = [&](int rc) {
-        for (int q = 0; q < kPipeSlots; ++q)
-            if (pstream_[q]) (void)cudaStreamSynchronize(pstream_[q]);
-        (void)cudaGetLastError();
-        return rc;
-    };
+    // every early way out, an exception included, waits for the slots' streams
+    // first, so that no copy of this call is still in flight when the next call
+    // packs a slot
+    struct Settle {
+        const cudaStream_t* streams;
+        bool armed = true;
+        ~Settle() {
+            if (!armed) return;
+            for (int q = 0; q < kPipeSlots; ++q)
+                if (streams[q]) (void)cudaStreamSynchronize(streams[q]);
+            (void)cudaGetLastError();
+        }
+    } settle{pstream_};
     size_t k = 0, m = 0;
     for (size_t off = 0; off < count; off += m, ++k) {
         const int j = (int)(k % kPipeSlots);
-        if ((e = drain(j)) != cudaSuccess) return fail(cuda_error(e, "verify"));
-        if (const int rc = fault_point("verify launch")) return fail(rc);
+        if ((e = drain(j)) != cudaSuccess) return cuda_error(e, "verify");
+        if (const int rc = fault_point("verify launch")) return rc;
         m = chunks.size(k, count - off);
         const size_t o_p = m * 32, o_s = a16(o_p + m * pub_sz), o_o = o_s + m * 64;
         uint8_t* h = (uint8_t*)pstage_[j].p;
@@ -504,14 +509,15 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         const bool split = m >= kPackSplitItems;
         size_t copied = 0;
         auto field = [&](size_t at, const uint8_t* src, size_t width, size_t stride) -> cudaError_t {
-            parallel_copy(m, [&](size_t lo, size_t hi) {
+            const auto rows = [&](size_t lo, size_t hi) {
                 if (stride == width) {
                     stage_copy(h + at + lo * width, src + (off + lo) * width, (hi - lo) * width);
                 } else {
                     stage_rows(h + at + lo * width, src + (off + lo) * stride, width, stride, hi - lo);
                 }
                 stage_fence();
-            });
+            };
+            parallel_copy(m, std::cref(rows));
             if (!split && at != o_s) return cudaSuccess;
             size_t end = at + m * width;
             if (at == o_s && collect) {
@@ -525,21 +531,22 @@ int Backend::verify_host_strided(int kind, const uint8_t* msgs, size_t m_stride,
         NvtxRange pack_range("pack chunk");
         if ((e = field(0, msgs, 32, m_stride)) != cudaSuccess || (e = field(o_p, pubs, pub_sz, p_stride)) != cudaSuccess ||
             (e = field(o_s, sigs, 64, s_stride)) != cudaSuccess)
-            return fail(cuda_error(e, "host->device copy"));
+            return cuda_error(e, "host->device copy");
         if (chunks.after_previous(k, m) &&
             (e = cudaStreamWaitEvent(pstream_[j], pev_[(k - 1) % kPipeSlots], 0)) != cudaSuccess)
-            return fail(cuda_error(e, "event wait"));
+            return cuda_error(e, "event wait");
         e = launch_verify(kind, d, d + o_p, d + o_s, (uint32_t)m, d + o_o, collect, pstream_[j], count);
-        if (e != cudaSuccess) return fail(cuda_error(e, "verify launch"));
+        if (e != cudaSuccess) return cuda_error(e, "verify launch");
         if ((e = cudaMemcpyAsync(h + o_o, d + o_o, m, cudaMemcpyDeviceToHost, pstream_[j])) != cudaSuccess)
-            return fail(cuda_error(e, "device->host copy"));
-        if ((e = cudaEventRecord(pev_[j], pstream_[j])) != cudaSuccess) return fail(cuda_error(e, "event record"));
+            return cuda_error(e, "device->host copy");
+        if ((e = cudaEventRecord(pev_[j], pstream_[j])) != cudaSuccess) return cuda_error(e, "event record");
         pend_off[j] = off;
         pend_n[j] = m;
         pend_out[j] = o_o;
     }
     for (int j = 0; j < kPipeSlots; ++j)
-        if ((e = drain(j)) != cudaSuccess) return fail(cuda_error(e, "verify"));
+        if ((e = drain(j)) != cudaSuccess) return cuda_error(e, "verify");
+    settle.armed = false;
     clear_error();
     return kOk;
 }
@@ -644,8 +651,8 @@ int Backend::verify_jobs(const VerifyJob* jobs, size_t n_jobs, uint32_t rlc_segm
 void Backend::parallel_copy(size_t n, const std::function<void(size_t, size_t)>& fn) {
     if (n < kPackSplitItems) return fn(0, n);
     // pieces are taken one at a time: a helper that wakes late takes fewer
-    parallel_run((int)((n + kPackPiece - 1) / kPackPiece),
-                 [&](int p) { fn(p * kPackPiece, std::min(n, (p + 1) * kPackPiece)); });
+    const auto piece = [&](int p) { fn(p * kPackPiece, std::min(n, (p + 1) * kPackPiece)); };
+    parallel_run((int)((n + kPackPiece - 1) / kPackPiece), std::cref(piece));
 }
 
 void Backend::parallel_run(int parts, const std::function<void(int)>& fn) {

@@ -218,7 +218,9 @@ private:
 
 public:
     // fn(lo, hi) over [0, n) split between the staging-copy threads (the
-    // caller included) when n is large enough to pay for them.
+    // caller included) when n is large enough to pay for them.  A callable passed
+    // by std::cref is not copied: no allocation, so nothing throws in the middle of
+    // a call.
     void parallel_copy(size_t n, const std::function<void(size_t, size_t)>& fn);
     // fn(part) for every part in [0, parts) on those threads.
     void parallel_run(int parts, const std::function<void(int)>& fn);
