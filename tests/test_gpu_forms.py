@@ -1,0 +1,106 @@
+"""Kernel forms that other tests' sizes do not force: the per-thread kernels with the
+key table where some lanes find their key and some do not, bucket chunks of every
+kind in a multi-scalar multiplication, the two main kernels on the same items."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import ultrafastsecp256k1_b200 as uf
+from conftest import ecdsa_corpus, msm_corpus, schnorr_corpus
+from test_gpu_keytable import _check, _jobs, _keyed_corpus
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def thread_ctx():
+    """A context whose mixed jobs and served launches of every size take a thread per signature."""
+    with uf.GpuContext(0) as ctx:
+        for k in (0, 1):
+            ctx.set_lanes(k, 1)
+        yield ctx
+
+
+@pytest.fixture(scope="module")
+def many_keys(oracle):
+    """2,000 distinct keys, each in a few items, with every key edge case."""
+    e = _keyed_corpus(oracle, 0, 2500, 1000, seed=621)
+    s = _keyed_corpus(oracle, 1, 2500, 1000, seed=622)
+    return e, s, oracle.ecdsa_verify_batch(*e), oracle.schnorr_verify_batch(*s)
+
+
+def test_lanes_with_and_without_a_table(thread_ctx, many_keys):
+    """256 slots: most lanes build their key's table beside lanes that copy one."""
+    e, s, we, ws = many_keys
+    jobs = _jobs(e, s, cut=300)
+    thread_ctx.set_key_table(8)
+    for _ in range(2):
+        _check(thread_ctx.verify_jobs(jobs), jobs, we, ws)
+    st = thread_ctx.key_table_stats()
+    assert st["slots"] == 256 and 0 < st["hits"] < st["lookups"]
+
+
+def test_full_blocks_with_and_without_a_table(thread_ctx, many_keys):
+    """The same above a half block per SM (256-thread blocks)."""
+    e, s, we, ws = many_keys
+    rng = np.random.default_rng(5)
+    oe, os_ = rng.integers(0, len(we), 19500), rng.integers(0, len(ws), 19500)
+    jobs = [(0, *(np.ascontiguousarray(a[oe]) for a in e)), (1, *(np.ascontiguousarray(a[os_]) for a in s))]
+    for log2 in (8, 16, 16):
+        thread_ctx.set_key_table(log2)
+        for _ in range(2):
+            got = thread_ctx.verify_jobs(jobs)
+            assert (got[0] == we[oe]).all() and (got[1] == ws[os_]).all()
+
+
+def test_served_launches_read_the_table(thread_ctx, many_keys):
+    """A burst submitted before any wait, twice over, with a table that overflows and one that does not."""
+    e, s, we, ws = many_keys
+    jobs = _jobs(e, s, cut=200)
+    for log2 in (8, 14):
+        with uf.Server(thread_ctx, slots=4, key_cache_log2=log2) as srv:
+            for _ in range(2):
+                ids = [srv.submit([j]) for j in jobs]
+                _check([srv.wait(i)[0] for i in ids], jobs, we, ws)
+            st = srv.stats()
+            assert 0 < st["cache_hits"] < st["cache_lookups"]
+
+
+@pytest.mark.parametrize("chunk", [2, 24, 256])
+def test_equal_and_opposite_points_by_chunk(oracle, chunk):
+    """P + P and P + (-P) inside one chunk (256), between a bucket's few chunks (24)
+    and between the many chunks of a heavy bucket (2)."""
+    L = uf.load_library()
+    L.ufsecp_gpu_msm.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_size_t, ctypes.c_void_p]
+    ks, pts = msm_corpus(oracle, 8, seed=85)
+    neg = pts.copy()
+    neg[:, 0] ^= 1
+    cases = [(np.repeat(ks[:1], 60, 0), np.repeat(pts[:1], 60, 0)),
+             (np.concatenate([np.repeat(ks[:1], 60, 0), ks[3:4]]),
+              np.concatenate([np.repeat(pts[:1], 30, 0), np.repeat(neg[:1], 30, 0), pts[3:4]])),
+             (np.repeat(ks[:1], 300, 0), np.concatenate([pts[:1], neg[:1]] * 150)),
+             (np.repeat(ks[:1], 301, 0), np.concatenate([pts[:1], neg[:1]] * 150 + [pts[:1]]))]
+    with uf.GpuContext(0) as ctx:
+        ctx.set_rlc_chunk(chunk)
+        for k, p in cases:
+            k, p = np.ascontiguousarray(k), np.ascontiguousarray(p)
+            out = np.full(33, 7, np.uint8)
+            rc = L.ufsecp_gpu_msm(ctx.handle, k.ctypes.data, p.ctypes.data, len(k), out.ctypes.data)
+            st, want = oracle.msm(k, p)
+            assert (rc, out.tobytes()) == (st, want)
+
+
+@pytest.mark.parametrize("n", [300, 20011, 50021])
+def test_integer_and_fp64_kernels_agree(oracle, n):
+    em, ep, es = ecdsa_corpus(oracle, 701, 31)
+    sm, sp, ss = schnorr_corpus(oracle, 701, 32, tamper=0.1)
+    we, ws = oracle.ecdsa_verify_batch(em, ep, es), oracle.schnorr_verify_batch(sm, sp, ss)
+    order = np.random.default_rng(n).integers(0, 701, n)
+    with uf.GpuContext(0) as ctx:
+        for group in (1, 128):
+            for k in (0, 1):
+                ctx.set_lanes(k, 1)
+                ctx.set_inversion_group(k, group)
+            assert (ctx.ecdsa_verify_batch(em[order], ep[order], es[order]) == we[order]).all()
+            assert (ctx.schnorr_verify_batch(sm[order], sp[order], ss[order]) == ws[order]).all()
