@@ -42,11 +42,11 @@ struct RlcSeed {
 
 // Lanes per window sum (a power of two), each over B / S buckets: about the
 // square root of B where the windows fill the device, more (up to 256, down to
-// four buckets a lane) while twice as many still leave it at two warps per
-// scheduler.
-inline int window_lanes(int c, uint64_t windows) {
+// four buckets a lane) while twice as many still leave it at two warps on each
+// of the device's schedulers (four per SM).
+inline int window_lanes(int c, uint64_t windows, int schedulers) {
     int S = c >= 9 ? 32 : 1 << ((c - 1) / 2);
-    while (S < 256 && 8 * S <= 1 << (c - 1) && 2 * S * windows <= 2 * 592 * 32) S *= 2;
+    while (S < 256 && 8 * S <= 1 << (c - 1) && 2 * S * windows <= 2ull * schedulers * 32) S *= 2;
     return S;
 }
 
@@ -779,7 +779,7 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     int mag_bits = 129;
     if (locate)
         for (uint32_t v = maxlen; v; v >>= 1) ++mag_bits;
-    const int W = (mag_bits + c - 1) / c, B = 1 << (c - 1), S = window_lanes(c, (uint64_t)n_seg * W);
+    const int W = (mag_bits + c - 1) / c, B = 1 << (c - 1), S = window_lanes(c, (uint64_t)n_seg * W, be_->sms() * 4);
     std::vector<uint32_t> host(3 * (size_t)n_seg + 1);
     uint64_t total = 0;
     for (uint32_t k = 0; k < n_seg; ++k) {
@@ -792,8 +792,8 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     host[3 * (size_t)n_seg] = (uint32_t)total;
     const uint64_t K = (uint64_t)n_seg * W * B;
     if (K >= 0x7FFFFFFFull) return be_->set_error(kErrBadInput, "RLC round too large");
-    // A round of few entries is cut finer than tuned, to about two chunks per
-    // thread of the device: 8,192 items in one batch 2.0 ms with chunks of 96,
+    // A round of few entries is cut finer than tuned, to about a chunk per
+    // resident thread of k_rlc_chunks (two blocks of 128 on each SM): 8,192 items in one batch 2.0 ms with chunks of 96,
     // 1.7 with 24; 262,144 at 4,096 per batch 4.6 with 8, 4.3 with 48 - 96.
     uint32_t chunk = be_->rlc_chunk(maxlen);
     if (!be_->rlc_chunk_fixed())
@@ -865,7 +865,7 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
                                 (uint32_t*)heavy_.p, be_->sms() * 4, s);
     if (e != cudaSuccess) return be_->cuda_error(e, "RLC bucket merge");
     e = launch_rlc_windows(g, (const uint4*)buckets_.p, (uint4*)wins_.p, (const uint32_t*)segbad_.p,
-                           (uint8_t*)segok_.p, (uint4*)segpt_.p, s);
+                           (uint8_t*)segok_.p, (uint4*)segpt_.p, be_->sms() * 4, s);
     if (e == cudaSuccess) e = cudaGetLastError();
     ok.resize(n_seg);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ok.data(), segok_.p, n_seg, cudaMemcpyDeviceToHost, s);

@@ -27,13 +27,6 @@ __device__ __forceinline__ void load_aff(const uint4* q, Fe& x, Fe& y) {
 // Jacobian point in global memory: X, Y, Z and the infinity flag (7 x uint4).
 constexpr int kJacQ = 7;
 
-__device__ __forceinline__ void store_jac(uint4* q, const Jac& P) {
-    store_aff(q, P.X, P.Y);
-    q[4] = make_uint4(P.Z.v[0], P.Z.v[1], P.Z.v[2], P.Z.v[3]);
-    q[5] = make_uint4(P.Z.v[4], P.Z.v[5], P.Z.v[6], P.Z.v[7]);
-    q[6] = make_uint4(P.inf ? 1u : 0u, 0u, 0u, 0u);
-}
-
 __device__ __forceinline__ void load_jac(const uint4* q, Jac& P) {
     load_aff(q, P.X, P.Y);
     const uint4 a = q[4], b = q[5];

@@ -183,12 +183,12 @@ inline unsigned grid_of(uint64_t n, int threads) { return (unsigned)((n + thread
 }  // namespace
 
 cudaError_t launch_rlc_windows(const RoundGeo& g, const uint4* buckets, uint4* wins, const uint32_t* segbad,
-                               uint8_t* segok, uint4* segpt, cudaStream_t s) {
+                               uint8_t* segok, uint4* segpt, int schedulers, cudaStream_t s) {
     const uint64_t n_seg = g.n_seg;
     const int threads = g.S > 32 ? g.S : 32;
     k_rlc_window<<<grid_of(n_seg * g.W * g.S, threads), threads, 0, s>>>(g, buckets, wins);
     int lanes = 32;                                // while the warps stay at one per scheduler
-    while (lanes > 1 && (n_seg * lanes > 592 * 32 || lanes >= 2 * g.W)) lanes >>= 1;
+    while (lanes > 1 && (n_seg * lanes > (uint64_t)schedulers * 32 || lanes >= 2 * g.W)) lanes >>= 1;
     k_rlc_finish<<<grid_of(n_seg * lanes, 32), 32, 0, s>>>(g, lanes, wins, segbad, segok, segpt);
     return cudaGetLastError();
 }

@@ -1,7 +1,5 @@
 // Launchers of the RLC kernels that run one serial chain per segment or
-// window (rlc_serial.cu): few threads, so latency-bound, and compiled with the
-// field and point operations inlined (the wide kernels of rlc.cu keep them out
-// of line for the instruction cache).
+// window (rlc_serial.cu): few threads, so latency-bound.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -13,9 +11,10 @@ namespace uf {
 // Running sums over each (segment, window)'s buckets in sub-ranges, their
 // combination per window, and Horner over the windows per segment:
 // segok[s] = 1 when segment s's sum is infinity, | 2 when it holds an item
-// that failed to parse; segpt[s] = the sum.
+// that failed to parse; segpt[s] = the sum.  schedulers: the device's, four per SM.
 cudaError_t launch_rlc_windows(const rlcdev::RoundGeo& g, const uint4* buckets, uint4* wins,
-                               const uint32_t* segbad, uint8_t* segok, uint4* segpt, cudaStream_t s);
+                               const uint32_t* segbad, uint8_t* segok, uint4* segpt, int schedulers,
+                               cudaStream_t s);
 
 // Buckets of two or more chunks: the sum of their chunk partials, by a thread
 // per bucket, or by a warp per bucket of more than kHeavyChunks chunks (their
