@@ -523,7 +523,7 @@ def bench_mixed(ctx, torch):
     group_items = 1 << 18
 
     def batched_pass():
-        # groups of consecutive batches packed into one persistent-queue launch;
+        # groups of consecutive batches packed into one mixed-job launch;
         # verdicts are compared after the timed loop
         got, exps = [], []
         t0 = _t.perf_counter()

@@ -36,9 +36,8 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_schnorr_verify_device(ufsecp_gpu_ctx* c
  * with the layouts of ufsecp_gpu_ecdsa_verify_batch (kind 0: 33-byte
  * compressed keys) or ufsecp_gpu_schnorr_verify_batch (kind 1: 32-byte x-only
  * keys), host buffers.  All jobs are packed into pinned staging and verified
- * by one persistent work-queue kernel (warps claim 32-item chunks from a
- * device queue head); layouts up to 65,536 items per kind replay a CUDA graph
- * captured per capacity bucket.  Synchronous, like the reference calls; the
+ * by one kernel launch per kind, side by side; layouts up to 65,536 items per
+ * kind replay a CUDA graph captured per capacity bucket.  Synchronous, like the reference calls; the
  * verdicts equal those of the per-kind calls item for item.  Kind 2 is
  * BIP-340 (the kind 1 layouts) checked by random linear combination: all
  * kind 2 items of the call are verified by one RLC batch verify (the
@@ -219,7 +218,7 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_schnorr_batch_identify_invalid(ufsecp_g
  * reference, which serves one synchronous call per batch).  A request is one
  * or more jobs (ECDSA and / or BIP-340, host buffers, layouts as above).
  * submit() returns at once with an id; a scheduler thread packs the oldest
- * pending requests into persistent-queue launches on `slots` streams as soon
+ * pending requests into mixed-job launches on `slots` streams as soon
  * as a slot and the memory budget allow (up to max_launch_items items per
  * launch; larger requests ride in several launches), so work that arrives
  * while other launches run overlaps with them on the device.  The request's
@@ -348,8 +347,9 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_device_props(ufsecp_gpu_ctx* ctx, int* 
  * read at context creation (UFSECP_B200_TUNING).  The tuning may also name a
  * small-launch variant per kind, used by verify calls of at most `items`
  * items (latency-bound launches with a few warps per SM, where inlining the
- * field arithmetic wins; the chunks of a larger call keep the main variant); set_variant applies its variant to every launch size and
- * clears the small-launch one.  get_small_variant reports -1 when none. */
+ * field arithmetic wins; the chunks of a larger call keep the main variant);
+ * set_variant applies its variant to every launch size and clears the
+ * small-launch one.  get_small_variant reports -1 when none. */
 #define UFSECP_EXT_VERIFY_VARIANTS 12
 UFSECP_API ufsecp_error_t ufsecp_gpu_ext_set_variant(ufsecp_gpu_ctx* ctx, int kind, int variant);
 UFSECP_API ufsecp_error_t ufsecp_gpu_ext_get_variant(ufsecp_gpu_ctx* ctx, int kind, int* variant_out,
@@ -360,11 +360,12 @@ UFSECP_API ufsecp_error_t ufsecp_gpu_ext_get_small_variant(ufsecp_gpu_ctx* ctx, 
 UFSECP_API ufsecp_error_t ufsecp_gpu_ext_set_small_variant(ufsecp_gpu_ctx* ctx, int kind, int variant,
                                                            uint32_t items);
 
-/* Several threads per signature (kind 0 ECDSA, 1 BIP-340): with lanes = 2, calls
- * of at most `items` items cut each signature's work between threads (four warps
- * of a block work on 32 signatures, above 32 signatures per SM two warps): a
- * shorter verify latency for more arithmetic in all, which pays while the device
- * has idle capacity (small calls).  lanes = 1 turns it off.  The tuning file sets
+/* Several threads per signature (kind 0 ECDSA, 1 BIP-340): with lanes = 2,
+ * launches of at most `items` items cut each signature's work between threads
+ * (four warps of a block work on 32 signatures, above 32 signatures per SM two
+ * warps): a shorter verify latency for more arithmetic in all, which pays while
+ * the device has idle capacity.  A small call is one launch; the short last chunk
+ * or wave of a large one is a launch too.  lanes = 1 turns it off.  The tuning file sets
  * it per kind (ecdsa_pair_items / schnorr_pair_items); set_variant turns it off.
  * The opaque-row / column surfaces follow the ECDSA setting. */
 UFSECP_API ufsecp_error_t ufsecp_gpu_ext_set_lanes(ufsecp_gpu_ctx* ctx, int kind, int lanes, uint32_t items);

@@ -428,7 +428,8 @@ class GpuContext:
         return outs
 
     def set_inversion_group(self, kind: int, group: int):
-        """ufsecp_gpu_ext_set_inversion_group: 1, 64 or 128 threads share each inversion."""
+        """ufsecp_gpu_ext_set_inversion_group: 1 the integer kernels, 64 or 128 the FP64
+        kernel."""
         self._check(self.L.ufsecp_gpu_ext_set_inversion_group(self._ctx, kind, group), "set_inversion_group")
 
     def get_inversion_group(self, kind: int) -> int:

@@ -8,7 +8,7 @@ arithmetic is inlined, i.e. instruction-cache footprint against call
 overhead, 9..11 in the P / G window widths: 3 / 18, 5 / 20, 4 / 16 bits
 against the default 4 / 20) on a GPU-signed batch, checks that all variants return identical
 verdicts, and picks them, plus the main kernel ("inversion group" 1: that
-variant, 64 or 128: the FP64 kernel), where the variant stays the main kernel a
+variant, 128: the FP64 kernel), where the variant stays the main kernel a
 small-launch variant and its item limit for latency-bound launches (a few warps
 per SM), and the launch size up to which four or two warps per 32 signatures beat
 a thread each; then, for RLC batch verification, it times the
@@ -130,12 +130,12 @@ def tune_lanes(ctx, torch, kind, bufs, reps: int = 10) -> dict:
     return {"items": items, "sigs_per_s": {str(l): {str(n): r for n, r in rs.items()} for l, rs in rates.items()}}
 
 
-INV_GROUPS = (1, 64, 128)
+INV_GROUPS = (1, 128)
 
 
 def tune_inversion_group(ctx, torch, kind, bufs, n, ref, reps: int = 3) -> dict:
     """Main kernel (ufsecp_gpu_ext_set_inversion_group): 1 (the tuned integer
-    variant) or 64 / 128 (the FP64 kernel), timed at the main batch size; each
+    variant) or 128 (the FP64 kernel), timed at the main batch size; each
     must reproduce the verdicts."""
     rates = {}
     for g in INV_GROUPS:

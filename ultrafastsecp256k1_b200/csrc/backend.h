@@ -79,7 +79,7 @@ public:
     // Batch signing (workload generator), device buffers, asynchronous.
     int sign_device(int kind, const uint8_t* d_msgs, const uint8_t* d_sks, const uint8_t* d_auxs, size_t count,
                     uint8_t* d_pubs, uint8_t* d_sigs, uint8_t* d_ok, cudaStream_t stream);
-    // Mixed ECDSA / BIP-340 jobs (host buffers) in one persistent-queue launch;
+    // Mixed ECDSA / BIP-340 jobs (host buffers), a verify kernel per kind side by side;
     // synchronous.  Keys go through the context's resident key table when it
     // is on (set_key_table).  Kind 2 jobs (BIP-340 by RLC) are verified after
     // the others by the RLC verifier, all in one batch of `rlc_segment`-item

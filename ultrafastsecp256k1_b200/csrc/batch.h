@@ -43,7 +43,7 @@ public:
     BatchSlot(const BatchSlot&) = delete;
     BatchSlot& operator=(const BatchSlot&) = delete;
 
-    // Creates the stream, completion event and queue head on the backend's device.
+    // Creates the streams, the events and the graphs' staging on the backend's device.
     int init(Backend* be, bool use_graphs = true);
     // Packs `jobs` and enqueues the work; returns immediately.  The jobs' host
     // buffers must stay valid until finish() returns.  in_flight: items that

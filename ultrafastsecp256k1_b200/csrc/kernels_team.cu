@@ -46,7 +46,7 @@ cudaError_t launch_verify_team(int kind, const uint8_t* msgs, const uint8_t* pub
     const uint4* comb = reinterpret_cast<const uint4*>(d_comb);
     // more than a block per SM: two warps per 32 signatures, so that a second
     // block still finds idle schedulers (6,011 signatures 440 us by four warps, 338
-    // by two; up to a block per SM 286 by four)
+    // by two; up to a block per SM 269 by four)
     if (n > (uint32_t)sms * kTeamLanes) launch_team<2>(kind, msgs, pubs, sigs, n, gt, comb, out, collect, s);
     else launch_team<4>(kind, msgs, pubs, sigs, n, gt, comb, out, collect, s);
     return cudaGetLastError();

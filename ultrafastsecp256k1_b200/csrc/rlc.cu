@@ -793,8 +793,9 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     const uint64_t K = (uint64_t)n_seg * W * B;
     if (K >= 0x7FFFFFFFull) return be_->set_error(kErrBadInput, "RLC round too large");
     // A round of few entries is cut finer than tuned, to about a chunk per
-    // resident thread of k_rlc_chunks (two blocks of 128 on each SM): 8,192 items in one batch 2.0 ms with chunks of 96,
-    // 1.7 with 24; 262,144 at 4,096 per batch 4.6 with 8, 4.3 with 48 - 96.
+    // resident thread of k_rlc_chunks (two blocks of 128 on each SM): 8,192 items
+    // in one batch 2.0 ms with chunks of 96, 1.7 with 24; 262,144 at 4,096 per
+    // batch 4.6 with 8, 4.3 with 48 - 96.
     uint32_t chunk = be_->rlc_chunk(maxlen);
     if (!be_->rlc_chunk_fixed())
         chunk = std::min(chunk, std::max(24u, (uint32_t)(total / ((uint64_t)be_->sms() * 256))));
@@ -838,8 +839,9 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
         k_rlc_scale<<<dim3(n_seg, (maxlen + 255) / 256), 256, 0, s>>>(d_seg, (const uint4*)mags_.p,
                                                                       (const RlcItem*)items_.p, (uint4*)lmags_.p,
                                                                       (uint32_t*)lmags_hi_.p);
-    k_rlc_tsum<<<n_seg, maxlen > 2048 ? kTsumThreads : 256, 0, s>>>(g, (const uint32_t*)tsc_.p, (const uint8_t*)okb_.p, (uint4*)segmag_.p,
-                                     (uint8_t*)segneg_.p, (uint32_t*)segbad_.p, locate ? 1 : 0);
+    k_rlc_tsum<<<n_seg, maxlen > 2048 ? kTsumThreads : 256, 0, s>>>(
+        g, (const uint32_t*)tsc_.p, (const uint8_t*)okb_.p, (uint4*)segmag_.p, (uint8_t*)segneg_.p,
+        (uint32_t*)segbad_.p, locate ? 1 : 0);
     uint32_t* ranks = (uint32_t*)cursor_.p;
     k_rlc_digits<<<grid_for(total / (size_t)W, 256), 256, 0, s>>>(g, mags, mags_hi, (const uint4*)segmag_.p,
                                                                  (const uint8_t*)segneg_.p, (uint32_t)total, counts,

@@ -6,7 +6,7 @@
 // and return at once with an id.  One scheduler thread owns `slots` batch
 // slots (each its own stream, pinned staging and CUDA graphs, batch.h):
 // whenever a slot is free it packs the oldest pending requests, up to
-// max_launch_items items, into one persistent-queue launch, so requests that
+// max_launch_items items, into one mixed-job launch, so requests that
 // arrive while others run are admitted as soon as a slot and memory free up,
 // and their launches overlap on the device.  A request larger than
 // max_launch_items is cut into pieces that ride in successive launches.

@@ -6,7 +6,7 @@
 
 Each case signs its own seeded BIP-340 / ECDSA corpus on the GPU, runs the
 named path R times on device-resident inputs (the plain per-signature kernel,
-the RLC batch verifier, or the mixed-job work-queue kernel), checks every
+the RLC batch verifier, or the mixed-job kernels), checks every
 verdict against the construction (valid signatures, plus one flipped bit in a
 known set) and prints one line of timings.  The cases hold well under 1 GB on
 the device, so a profiler capture of them stays small.
