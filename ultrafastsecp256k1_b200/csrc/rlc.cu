@@ -863,8 +863,8 @@ int RlcVerifier::run_round(const std::vector<uint32_t>& seg, int c, cudaStream_t
     k_rlc_chunks<<<grid_for(chunk_cap, kChunkThreads), kChunkThreads, 0, s>>>(
         coff, (uint32_t)K, (const uint4*)crec_.p, (const uint32_t*)entries_.p, (const RlcItem*)items_.p, 3u * n_,
         (const uint4*)be_->gtab(), (uint4*)partials_.p, (uint4*)buckets_.p);
-    e = launch_rlc_bucket_merge(coff, (uint32_t)K, (const uint4*)partials_.p, (uint4*)buckets_.p,
-                                (uint32_t*)heavy_.p, be_->sms() * 4, s);
+    e = launch_rlc_bucket_merge(coff, (uint32_t)K, heavy_chunks(total, K, chunk), (const uint4*)partials_.p,
+                                (uint4*)buckets_.p, (uint32_t*)heavy_.p, be_->sms() * 4, s);
     if (e != cudaSuccess) return be_->cuda_error(e, "RLC bucket merge");
     e = launch_rlc_windows(g, (const uint4*)buckets_.p, (uint4*)wins_.p, (const uint32_t*)segbad_.p,
                            (uint8_t*)segok_.p, (uint4*)segpt_.p, be_->sms() * 4, s);

@@ -130,7 +130,7 @@ k_rlc_finish(RoundGeo g, int lanes, const uint4* __restrict__ wins, const uint32
 }
 
 // Buckets with 0 or >= 2 chunks: infinity, or the sum of their partials.
-// A bucket of more than kHeavyChunks chunks (skewed digits: the top windows
+// A bucket of more than heavy_from chunks (skewed digits: the top windows
 // of a locate round's j-scaled magnitudes put most points of a segment into a
 // few buckets) is left to k_rlc_bucket_heavy: its key goes to `heavy`.
 __device__ __forceinline__ void add_partial(JacD& acc, const uint4* q) {
@@ -140,13 +140,13 @@ __device__ __forceinline__ void add_partial(JacD& acc, const uint4* q) {
 }
 
 __global__ void __launch_bounds__(128)
-k_rlc_bucket_fin(const uint32_t* __restrict__ coff, uint32_t K, const uint4* __restrict__ partials,
-                 uint4* __restrict__ buckets, uint32_t* __restrict__ heavy) {
+k_rlc_bucket_fin(const uint32_t* __restrict__ coff, uint32_t K, uint32_t heavy_from,
+                 const uint4* __restrict__ partials, uint4* __restrict__ buckets, uint32_t* __restrict__ heavy) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
     const uint32_t c0 = coff[k], c1 = coff[k + 1];
     if (c1 - c0 == 1) return;
-    if (c1 - c0 > kHeavyChunks) {
+    if (c1 - c0 > heavy_from) {
         heavy[1 + atomicAdd(&heavy[0], 1u)] = k;
         return;
     }
@@ -193,9 +193,9 @@ cudaError_t launch_rlc_windows(const RoundGeo& g, const uint4* buckets, uint4* w
     return cudaGetLastError();
 }
 
-cudaError_t launch_rlc_bucket_merge(const uint32_t* coff, uint32_t K, const uint4* partials, uint4* buckets,
-                                    uint32_t* heavy, int heavy_grid, cudaStream_t s) {
-    k_rlc_bucket_fin<<<grid_of(K, 128), 128, 0, s>>>(coff, K, partials, buckets, heavy);
+cudaError_t launch_rlc_bucket_merge(const uint32_t* coff, uint32_t K, uint32_t heavy_from, const uint4* partials,
+                                    uint4* buckets, uint32_t* heavy, int heavy_grid, cudaStream_t s) {
+    k_rlc_bucket_fin<<<grid_of(K, 128), 128, 0, s>>>(coff, K, heavy_from, partials, buckets, heavy);
     k_rlc_bucket_heavy<<<heavy_grid, 128, 0, s>>>(coff, partials, buckets, heavy);
     return cudaGetLastError();
 }

@@ -17,9 +17,9 @@ cudaError_t launch_rlc_windows(const rlcdev::RoundGeo& g, const uint4* buckets, 
                                cudaStream_t s);
 
 // Buckets of two or more chunks: the sum of their chunk partials, by a thread
-// per bucket, or by a warp per bucket of more than kHeavyChunks chunks (their
-// keys listed in heavy[1..heavy[0]] by the first kernel).
-cudaError_t launch_rlc_bucket_merge(const uint32_t* coff, uint32_t K, const uint4* partials, uint4* buckets,
-                                    uint32_t* heavy, int heavy_grid, cudaStream_t s);
+// per bucket, or by a warp per bucket of more than heavy_from >= kHeavyChunks
+// chunks (their keys listed in heavy[1..heavy[0]] by the first kernel).
+cudaError_t launch_rlc_bucket_merge(const uint32_t* coff, uint32_t K, uint32_t heavy_from, const uint4* partials,
+                                    uint4* buckets, uint32_t* heavy, int heavy_grid, cudaStream_t s);
 
 }  // namespace uf
