@@ -92,6 +92,23 @@ def test_equal_and_opposite_points_by_chunk(oracle, chunk):
             assert (rc, out.tobytes()) == (st, want)
 
 
+def test_server_captures_one_form_a_shape():
+    """A server whose small launches have three forms starts as fast as one whose launches
+    have one: as many graphs each, within a quarter for the host's noise."""
+    with uf.GpuContext(0) as one, uf.GpuContext(0) as three:
+        best = {}
+        for ctx, lanes in ((one, 1), (three, 2)):
+            for k in (0, 1):
+                ctx.set_lanes(k, lanes, 9472)
+        for _ in range(8):
+            for ctx in (one, three):
+                t = time.perf_counter()
+                srv = uf.Server(ctx)
+                best[ctx] = min(best.get(ctx, 1e9), time.perf_counter() - t)
+                srv.close()
+        assert best[three] <= 1.25 * best[one], list(best.values())
+
+
 @pytest.mark.parametrize("batch,chunk", [(512, 6), (1000, 8), (16384, 6)])
 def test_short_chunks_of_even_buckets(batch, chunk):
     """Chunks of a few entries, as tuning files of earlier builds hold, cut every bucket into

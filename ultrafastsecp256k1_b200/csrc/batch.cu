@@ -86,20 +86,24 @@ int BatchSlot::init(Backend* be, bool use_graphs) {
 }
 
 // Warps per 32 signatures of a small launch: four up to 32 items per SM, two up
-// to the backend's tuned limit (64 per SM), 0 (a thread each) above.  What other
-// slots have in flight counts too: sharing a signature halves a launch's time on
-// an idle device (0.29 against 0.54 ms) and costs rate on a busy one (a burst of
-// 96 requests, 47,000 signatures: 2.7 ms with four warps in every small launch,
-// 2.4 ms with them only up to the limits in flight).  The choice is part of the
-// graph key, so a graph captured with the other kernels is never replayed.
-int BatchSlot::team_warps(const QueueArgs& a) const {
+// to the backend's tuned limit (64 per SM), 0 (a thread each) above.  `beside`:
+// what other slots have in flight counts too, since sharing a signature halves a
+// launch's time on an idle device (0.29 against 0.54 ms) and costs rate on a busy
+// one (a burst of 96 requests, 47,000 signatures: 2.7 ms with four warps in every
+// small launch, 2.4 ms with them only up to the limits in flight).
+int BatchSlot::team_warps(const QueueArgs& a, uint64_t beside) const {
     const uint64_t limit = be_->queue_pair_items();
-    const uint64_t items = std::max((uint64_t)a.cap_e + a.cap_s, beside_);
+    const uint64_t items = std::max((uint64_t)a.cap_e + a.cap_s, beside);
     return items > limit ? 0 : (items > (uint64_t)be_->sms() * 32 ? 2 : 4);
 }
 
+// Graphs hold the form of a launch alone on the device; the form is in the key
+// because the tuned limit may change.  A launch that takes another form beside other
+// slots' work is issued step by step: as fast there (96 requests 2.28 ms, 2.31 with
+// graphs of every form), and a server captures 99 graphs a slot instead of 172 (177
+// ms to create one with eight slots, 375 before).
 uint64_t BatchSlot::graph_key(const QueueArgs& a) const {
-    return ((uint64_t)a.cap_e << 32) | a.cap_s | ((uint64_t)team_warps(a) << 61);
+    return ((uint64_t)a.cap_e << 32) | a.cap_s | ((uint64_t)team_warps(a, 0) << 61);
 }
 
 QueueArgs BatchSlot::args_for(uint8_t* d) const {
@@ -127,12 +131,12 @@ QueueArgs BatchSlot::args_for(uint8_t* d) const {
     return a;
 }
 
-int BatchSlot::run_direct(const QueueArgs& a) {
+int BatchSlot::run_direct(const QueueArgs& a, int warps) {
     uint8_t* h = staged_big_ ? (uint8_t*)big_pinned_.p : (uint8_t*)pinned_.p;
     uint8_t* d = staged_big_ ? (uint8_t*)big_dev_.p : (uint8_t*)dev_.p;
     cudaError_t e = cudaMemcpyAsync(d, h, layout_.in_bytes, cudaMemcpyHostToDevice, stream_);
     if (e == cudaSuccess)
-        e = launch_verify_queue(a, team_warps(a), be_->gtab(), be_->comb(), be_->sms(),
+        e = launch_verify_queue(a, warps, be_->gtab(), be_->comb(), be_->sms(),
                                 QueueStreams{stream_, stream2_, stream3_, fork_, join_, join3_});
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h + layout_.e_out, d + layout_.e_out, layout_.out_bytes, cudaMemcpyDeviceToHost, stream_);
@@ -140,14 +144,15 @@ int BatchSlot::run_direct(const QueueArgs& a) {
     return kOk;
 }
 
-int BatchSlot::run_graph(const QueueArgs& a, uint64_t key) {
+int BatchSlot::graph_for(const QueueArgs& a, cudaGraphExec_t* out) {
+    const uint64_t key = graph_key(a);
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
         cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
         cudaError_t e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return be_->cuda_error(e, "graph capture");
-        const int rc = run_direct(a);
+        const int rc = run_direct(a, team_warps(a, 0));
         e = cudaStreamEndCapture(stream_, &g);
         if (rc != kOk) {
             if (g) cudaGraphDestroy(g);
@@ -158,7 +163,14 @@ int BatchSlot::run_graph(const QueueArgs& a, uint64_t key) {
         if (e != cudaSuccess) return be_->cuda_error(e, "graph instantiate");
         it = graphs_.emplace(key, exec).first;
     }
-    cudaError_t e = cudaGraphLaunch(it->second, stream_);
+    *out = it->second;
+    return kOk;
+}
+
+int BatchSlot::run_graph(const QueueArgs& a) {
+    cudaGraphExec_t exec = nullptr;
+    if (const int rc = graph_for(a, &exec)) return rc;
+    const cudaError_t e = cudaGraphLaunch(exec, stream_);
     if (e != cudaSuccess) return be_->cuda_error(e, "graph launch");
     return kOk;
 }
@@ -222,7 +234,7 @@ int BatchSlot::enqueue(const VerifyJob* jobs, size_t n_jobs, size_t in_flight) {
     if (const int rc = be_->fault_point("batch enqueue")) return rc;
     size_t n_e = 0, n_s = 0;
     for (size_t j = 0; j < n_jobs; ++j) (jobs[j].kind == 0 ? n_e : n_s) += jobs[j].count;
-    beside_ = in_flight ? in_flight + n_e + n_s : 0;
+    const uint64_t beside = in_flight ? in_flight + n_e + n_s : 0;
     cudaError_t e = cudaSetDevice(be_->device());
     if (e != cudaSuccess) return be_->cuda_error(e, "cudaSetDevice");
     // the staging is reused: the previous launch (finished or abandoned after
@@ -246,9 +258,13 @@ int BatchSlot::enqueue(const VerifyJob* jobs, size_t n_jobs, size_t in_flight) {
     pack(jobs, n_jobs, h, parallel_pack_ && n_e + n_s >= kParallelPackItems);
     uint8_t* d = staged_big_ ? (uint8_t*)big_dev_.p : (uint8_t*)dev_.p;
     const QueueArgs a = args_for(d);
-    last_graph_ = graph;
-    const int rc = graph ? run_graph(a, graph_key(a)) : run_direct(a);
-    if (rc != kOk) return rc;
+    last_graph_ = graph && team_warps(a, beside) == team_warps(a, 0);
+    const int rc = last_graph_ ? run_graph(a) : run_direct(a, team_warps(a, beside));
+    if (rc != kOk) {
+        // part of the launch may be in flight: the staging is packed again next
+        for (cudaStream_t st : {stream_, stream2_, stream3_}) (void)cudaStreamSynchronize(st);
+        return rc;
+    }
     if ((e = cudaEventRecord(done_, stream_)) != cudaSuccess) return be_->cuda_error(e, "event record");
     return kOk;
 }
@@ -257,6 +273,7 @@ int BatchSlot::prewarm(uint32_t max_items) {
     if (!use_graphs_) return kOk;
     std::vector<uint32_t> caps = {0};
     for (uint32_t b = kMinBucket; b <= kGraphMaxItems; b <<= 1) caps.push_back(b);
+    uint32_t launched = 0;
     cudaError_t e = cudaSetDevice(be_->device());
     if (e != cudaSuccess) return be_->cuda_error(e, "cudaSetDevice");
     for (uint32_t ce : caps) {
@@ -269,11 +286,14 @@ int BatchSlot::prewarm(uint32_t max_items) {
             hdr[1] = 0;
             hdr[2] = 0;
             const QueueArgs a = args_for((uint8_t*)dev_.p);
-            for (const uint64_t beside : {(uint64_t)0, (uint64_t)be_->queue_pair_items(), ~(uint64_t)0}) {   // every form
-                beside_ = beside;
-                const int rc = run_graph(a, graph_key(a));
-                if (rc != kOk) return rc;
-            }
+            cudaGraphExec_t exec = nullptr;
+            if (const int rc = graph_for(a, &exec)) return rc;
+            // launched once per form and kinds, for its kernels: a graph's copies are as
+            // large as its buckets
+            const int form = team_warps(a, 0) * 4 + (ce ? 2 : 0) + (cs ? 1 : 0);
+            e = (launched >> form) & 1 ? cudaGraphUpload(exec, stream_) : cudaGraphLaunch(exec, stream_);
+            launched |= 1u << form;
+            if (e != cudaSuccess) return be_->cuda_error(e, "prewarm");
         }
     }
     if ((e = cudaStreamSynchronize(stream_)) != cudaSuccess) return be_->cuda_error(e, "prewarm");

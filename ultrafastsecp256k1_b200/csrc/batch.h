@@ -49,9 +49,9 @@ public:
     // buffers must stay valid until finish() returns.  in_flight: items that
     // other slots have on the device at that time.
     int enqueue(const VerifyJob* jobs, size_t n_jobs, size_t in_flight = 0);
-    // Captures and runs (with zero items) the graph of every capacity bucket
-    // pair whose total is at most max_items, so that later launches of any
-    // shape find their graph instantiated and their kernels loaded.
+    // Captures the graph of every capacity bucket pair whose total is at most
+    // twice max_items and runs one per form (with zero items), so that later
+    // launches of any shape find their graph instantiated and their kernels loaded.
     int prewarm(uint32_t max_items);
     // True once the enqueued work has completed on the device.
     bool ready();
@@ -86,10 +86,11 @@ private:
     template <class F>
     void each_field(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, F fn);
     void pack(const VerifyJob* jobs, size_t n_jobs, uint8_t* h, bool parallel);
-    int run_direct(const QueueArgs& a);
-    int team_warps(const QueueArgs& a) const;
+    int run_direct(const QueueArgs& a, int warps);
+    int team_warps(const QueueArgs& a, uint64_t beside) const;
     uint64_t graph_key(const QueueArgs& a) const;
-    int run_graph(const QueueArgs& a, uint64_t key);
+    int graph_for(const QueueArgs& a, cudaGraphExec_t* out);   // captured when first asked for
+    int run_graph(const QueueArgs& a);
     QueueArgs args_for(uint8_t* dev_base) const;
 
     Backend* be_ = nullptr;
@@ -107,7 +108,6 @@ private:
     bool staged_big_ = false;
     bool last_graph_ = false;
     bool parallel_pack_ = false;
-    uint64_t beside_ = 0;            // items on the device with this launch beside other slots' (0: alone)
     std::vector<Copy> copies_;       // the launch's staging copies, runs_[p] .. runs_[p + 1] one part
     std::vector<uint32_t> runs_;
     std::map<uint64_t, cudaGraphExec_t> graphs_;
